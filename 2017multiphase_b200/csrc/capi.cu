@@ -34,7 +34,7 @@ static int dalloc_t(MpCtx* c, T** p, size_t count) { return dalloc(c, (void**)p,
 static void free_all(MpCtx* c) {
     void* ptrs[] = {c->press, c->divg, c->lsfluid, c->lsair, c->lsmerge, c->phifluid, c->phiair, c->phisolid,
                     c->gx, c->gy, c->gz, c->gxa, c->gya, c->gza, c->sf, c->Tp, c->Tp_save, c->Tp_old, c->fixedheat,
-                    c->cell_tmp, c->mark, c->mark_tmp, c->cg_r, c->cg_p, c->cg_z, c->cg64, c->red, c->scal, c->red_count,
+                    c->cell_tmp, c->mark, c->mark_tmp, c->cg_r, c->cg_p, c->cg_z, c->cg64, c->cg_exch, c->red, c->scal, c->red_count,
                     c->pos, c->vel, c->heat, c->pos2, c->vel2, c->heat2, c->pdens, c->pprs, c->pscr, c->pscr2,
                     c->flag_snap, c->pflag8, c->pflag8s, c->keys, c->perm, c->cell_cnt, c->cell_off, c->tmask, c->air_brick, c->scan_tmp, c->u32_scratch,
                     c->randf, c->seeds, c->mc_numverts, c->mc_tri, c->mc_dens, c->mc_dens2, c->gfm_beta, c->gfm_s, c->mc_cube, c->mc_vflag, c->mc_vscan,
@@ -91,12 +91,16 @@ static int create_impl(MpCtx* c, const mp_params* p) {
     }
     MP_TRY(dalloc_t(c, &c->cg64, 5 * n));
     c->red_blocks = mp_blocks((long long)n, 256);
-    if (const char* e = getenv("MP_CG_KERNEL")) c->cg_use_tma = strcmp(e, "v4") != 0;
+    if (const char* e = getenv("MP_CG_KERNEL")) {
+        c->cg_use_tma = strcmp(e, "v4") != 0;
+        c->cg_use_res = c->cg_use_tma && strcmp(e, "tma") != 0;
+    }
     if (const char* e = getenv("MP_CG_TMA_CHUNK")) c->cg_tma_chunk = atoi(e);
     MP_TRY(dalloc_t(c, &c->red, (size_t)148 * 32 * 6));
     MP_TRY(dalloc_t(c, &c->scal, 16));
     MP_TRY(dalloc_t(c, &c->red_count, 16));
     MP_CUDA(c, cudaMemset(c->red_count, 0, 16 * sizeof(unsigned int)));
+    MP_TRY(k_cg_res_setup(c));
     MP_CUDA(c, cudaMemset(c->scal, 0, 16 * sizeof(double)));
     size_t cap = (size_t)std::max(p->par_num_max, 1);
     for (float4** f : {&c->pos, &c->vel, &c->heat, &c->pos2, &c->vel2, &c->heat2, &c->pscr, &c->pscr2})

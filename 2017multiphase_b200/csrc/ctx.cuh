@@ -22,6 +22,16 @@ struct McSurface {
     int nverts = 0, nindices = 0, active = 0;
 };
 
+// tiling of the on-chip CG solve (cg_res.cuh); nblk = 0: the grid does not fit
+struct ResGeom {
+    int ti, tj, nbi, nbj, KG;
+};
+struct ResPlan {
+    ResGeom g{};
+    int nblk = 0, Q = 0;
+    size_t smem = 0;
+};
+
 struct MpCtx {
     mp_params P{};
     mp_state S{};
@@ -55,9 +65,14 @@ struct MpCtx {
     unsigned int *red_count = 0; // last-block counters
     int red_blocks = 0;
     // CG kernels (tuning knobs read from the environment at mp_create):
-    // MP_CG_KERNEL=v4 keeps the float4-group passes where the TMA plane
+    // MP_CG_KERNEL=tma runs the passes one launch each where the on-chip solve
+    // applies, MP_CG_KERNEL=v4 the float4-group passes also where the TMA plane
     // marching applies; MP_CG_TMA_CHUNK sets its planes per CTA (0: derived)
-    int cg_use_tma = 1;
+    int cg_use_tma = 1, cg_use_res = 1;
+    ResPlan res_plan32, res_plan64;   // on-chip solve, FP32 and FP64 vectors
+    uint64_t* cg_exch = 0;            // its halo rows and partial sums
+    size_t cg_exch_words = 0;
+    uint32_t cg_epoch = 1;            // first tag that no exchange has used
     int cg_tma_chunk = 0;
     float *gfm_beta = 0;         // ghost-fluid face weights (x, y, z faces), allocated on first use
     float *gfm_s = 0;            // its Jacobi scaling per cell
@@ -205,6 +220,7 @@ int k_melt(MpCtx* c);
 int k_freeze(MpCtx* c);
 int k_mc(MpCtx* c, int surface);
 int k_mc_fluid_gas(MpCtx* c);
+int k_cg_res_setup(MpCtx* c);
 int k_cg_solve(MpCtx* c, const int8_t* mark, float* x, const float* b, int maxiter, int tolmode, float tol, int* iters,
                double* res);
 int k_cg_solve(MpCtx* c, const int8_t* mark, double* x, const double* b, int maxiter, int tolmode, float tol,

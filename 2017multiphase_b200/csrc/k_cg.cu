@@ -82,6 +82,25 @@ __device__ __forceinline__ bool finish_sum(const Red& R, double mine, double* to
 __device__ __forceinline__ bool inner(const Grid& g, int i, int j, int k) {
     return i > 0 && i < g.NX - 1 && j > 0 && j < g.NY - 1 && k > 0 && k < g.NZ - 1;
 }
+// s / h^2 by the reciprocal: with c = 1/h^2 rounded to nearest, q = s c and its
+// exact remainder s - q h^2 (one fused operation), q + c times the remainder is
+// the correctly rounded quotient (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990). The remainder is
+// exact for |s| above 4e-31 (FP32); below, the last bit may differ. Three
+// operations, where a division by a variable takes about 5 cycles of an SM per
+// warp and in FP64 a call (around which registers spilled).
+struct CgQuot {
+    float f = 0.0f, hf = 0.0f;    // 1/h^2 (0: h^2 too far from one, divide) and h^2
+    double d = 0.0, hd = 0.0;
+};
+__device__ __forceinline__ float cg_quot(float s, const CgQuot& c) {
+    const float q = s * c.f;
+    return fabsf(q) <= 3.4e38f ? __fmaf_rn(__fmaf_rn(-q, c.hf, s), c.f, q) : q;
+}
+__device__ __forceinline__ double cg_quot(double s, const CgQuot& c) {
+    const double q = s * c.d;
+    return fabs(q) <= 1.7e308 ? __fma_rn(__fma_rn(-q, c.hd, s), c.d, q) : q;
+}
 // computeAx_bubble (spray_k.cu:3423-3447): rows over FLUID and AIR cells;
 // with air = false, computeAx (spray_k.cu:2300-2322) of the single-phase
 // solve: rows over FLUID cells only, AIR cells a zero-pressure region
@@ -112,12 +131,21 @@ struct PressOp {
         return s / h2;
     }
     // the same row, piecewise, for the plane-marching kernels
+    static constexpr bool kTypedDiag = false;   // one diagonal for all cells
+    __device__ __forceinline__ int type(int) const { return 0; }
+    template <class R> __device__ __forceinline__ R diag(int) const { return (R)(-6.0f); }
     __device__ __forceinline__ bool fixed(int q) const { return mark[q] == MP_TYPEBOUNDARY; }
     template <class R> __device__ __forceinline__ R start(int, R c) const { return (R)(-6.0f) * c; }
     template <class R> __device__ __forceinline__ R comb(R s, R v) const { return s + v; }
+    CgQuot rec;   // 1 / h^2 in FP32 and FP64
     template <class R> __device__ __forceinline__ R finish(R s) const {
-        if (inv_h2 != 0.0f) return s * (R)inv_h2;
+        if (rec.f != 0.0f) return finish_rec<R>(s);
         return s / ((R)g.h * (R)g.h);
+    }
+    // the same when rec.f != 0 is known (no division, so no call, in the kernel)
+    template <class R> __device__ __forceinline__ R finish_rec(R s) const {
+        if (inv_h2 != 0.0f) return s * (R)inv_h2;
+        return cg_quot(s, rec);
     }
 };
 // PressOp with inv_h2 set when h^2 (rounded to float, as the stencil forms it)
@@ -125,6 +153,9 @@ struct PressOp {
 inline PressOp press_op(const Grid& g, const int8_t* mark, bool air = true) {
     PressOp op{g, mark, air};
     const float h2 = g.h * g.h;
+    op.rec.hf = h2;
+    op.rec.hd = (double)g.h * (double)g.h;
+    if (h2 > 1e-12f && h2 < 1e12f) { op.rec.f = 1.0f / h2; op.rec.d = 1.0 / op.rec.hd; }
     int e = 0;
     if (h2 > 0.0f && std::frexp(h2, &e) == 0.5f) op.inv_h2 = 1.0f / h2;
     return op;
@@ -167,14 +198,18 @@ struct HeatOp {
         q = idx - 1;  s -= fix(q) ? c : val(q);
         return s;
     }
-    __device__ __forceinline__ bool fixed(int q) const { return fix(q); }
-    template <class R> __device__ __forceinline__ R start(int idx, R c) const {
-        float al = al_of(mark[idx]);
+    static constexpr bool kTypedDiag = true;    // the diagonal goes by cell type
+    __device__ __forceinline__ int type(int idx) const { return mark[idx]; }
+    template <class R> __device__ __forceinline__ R diag(int t) const {
+        float al = al_of(t);
         float h = g.h;
-        return ((R)h * (R)h / (R)al / (R)dt + (R)6.0f) * c;
+        return (R)h * (R)h / (R)al / (R)dt + (R)6.0f;
     }
+    __device__ __forceinline__ bool fixed(int q) const { return fix(q); }
+    template <class R> __device__ __forceinline__ R start(int idx, R c) const { return diag<R>(mark[idx]) * c; }
     template <class R> __device__ __forceinline__ R comb(R s, R v) const { return s - v; }
     template <class R> __device__ __forceinline__ R finish(R s) const { return s; }
+    template <class R> __device__ __forceinline__ R finish_rec(R s) const { return s; }
 };
 
 // Ghost-fluid variable-density operator (the density-ratio extension; the
@@ -616,6 +651,7 @@ __global__ void __launch_bounds__(CG_T, 6) k_cg_v4(Op op, const uint8_t* __restr
 
 }  // namespace
 #include "cg_tma.cuh"
+#include "cg_res.cuh"
 namespace {
 
 // cptdivergence_bubble2 (spray_k.cu:3138-3263)
@@ -859,12 +895,96 @@ static Red red_of(MpCtx* c) {
     return Red{c->red, c->red_count, c->scal, reinterpret_cast<unsigned int*>(c->red_count + 1)};
 }
 
-// Runs CG on x (zeroed here) for A x = b. Batches iterations between host
+// The on-chip solve's plans and exchange buffer (cg_res.cuh), made once: the
+// grid of a context is fixed.
+int k_cg_res_setup(MpCtx* c) {
+    int sms = 0, smem = 0, coop = 0;
+    MP_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    MP_CUDA(c, cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    MP_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+    if (!coop || !c->cg_use_res) return MP_OK;
+    const size_t room = (size_t)smem - 1024;   // the kernel's static shared memory
+    c->res_plan32 = res_plan<float>(c->G, sms, room);
+    c->res_plan64 = res_plan<double>(c->G, sms, room);
+    const size_t words = std::max(c->res_plan32.nblk ? res_exch_words(c->res_plan32) : 0,
+                                  c->res_plan64.nblk ? res_exch_words(c->res_plan64) : 0);
+    if (!words) return MP_OK;
+    c->cg_exch_words = RES_SLOT_WORDS + words;
+    MP_CUDA(c, cudaMalloc((void**)&c->cg_exch, sizeof(uint64_t) * c->cg_exch_words));
+    MP_CUDA(c, cudaMemset(c->cg_exch, 0, sizeof(uint64_t) * c->cg_exch_words));
+    return MP_OK;
+}
+
+// The solve in one launch, when the grid fits on chip; *taken tells.
+template <class R, class Op>
+static int run_cg_res(MpCtx* c, const Op& op, R* x, const R* b, int maxiter, int tolmode, float tol, int* iters_out,
+                      double* res_out, int kt_class, bool* taken) {
+    const ResPlan& P = sizeof(R) == 4 ? c->res_plan32 : c->res_plan64;
+    *taken = P.nblk > 0 && maxiter < (1 << 28);
+    if (!*taken) return MP_OK;
+    void (*kern)(Op, ResGeom, const R*, R*, uint64_t*, uint64_t*, Red, int, float, int, uint32_t) = nullptr;
+    switch (P.Q) {
+    case 1: kern = k_cg_res<R, Op, 1>; break;
+    case 2: kern = k_cg_res<R, Op, 2>; break;
+    case 3: kern = k_cg_res<R, Op, 3>; break;
+    case 4: kern = k_cg_res<R, Op, 4>; break;
+    case 6: kern = k_cg_res<R, Op, 6>; break;
+    default: kern = k_cg_res<R, Op, 8>;
+    }
+    cudaStream_t s = c->stream;
+    Red Rd = red_of(c);
+    // tags run on from solve to solve; start over before they could wrap
+    if (c->cg_epoch > 0xffffffffu - 2u * (uint32_t)std::max(maxiter, 0) - 4u) {
+        MP_CUDA(c, cudaMemsetAsync(c->cg_exch, 0, sizeof(uint64_t) * c->cg_exch_words, s));
+        c->cg_epoch = 1;
+    }
+    MP_CUDA(c, cudaMemsetAsync(Rd.flag, 0xff, sizeof(unsigned int) * F_COUNT, s));
+    MP_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+    Op o = op;
+    ResGeom g = P.g;
+    uint64_t *slots = c->cg_exch, *exch = c->cg_exch + RES_SLOT_WORDS;
+    uint32_t epoch = c->cg_epoch;
+    void* args[] = {&o, &g, &b, &x, &exch, &slots, &Rd, &tolmode, &tol, &maxiter, &epoch};
+    {
+        KtScope kt(c, kt_class);
+        MP_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(P.nblk), dim3(RES_T), args,
+                                               P.smem, s));
+    }
+    c->launches++;
+    unsigned int hflag[F_COUNT] = {0, 0};
+    double rr = 0;
+    MP_CUDA(c, cudaMemcpyAsync(&rr, Rd.scal + S_RR, sizeof(double), cudaMemcpyDeviceToHost, s));
+    MP_CUDA(c, cudaMemcpyAsync(hflag, Rd.flag, sizeof(hflag), cudaMemcpyDeviceToHost, s));
+    MP_CUDA(c, cudaStreamSynchronize(s));
+    if (hflag[F_DONE] == DONE_TIMEOUT || hflag[F_DONE] == 0xffffffffu) {
+        MP_CUDA(c, cudaMemsetAsync(c->cg_exch, 0, sizeof(uint64_t) * c->cg_exch_words, s));
+        c->cg_epoch = 1;
+        c->err = "cg: an exchange between thread blocks ran out of time";
+        return MP_ERR_TIMEOUT;
+    }
+    c->cg_epoch += 2u * hflag[F_ITERS] + 4u;
+    *iters_out = (int)hflag[F_ITERS];
+    *res_out = rr;
+    c->work[MP_WC_CG_ITERS] += hflag[F_ITERS];
+    return hflag[F_DONE] == DONE_CAP ? MP_ERR_NOCONVERGE : MP_OK;
+}
+
+// Runs CG on x (zeroed here) for A x = b. Grids that fit on chip are solved in
+// one launch (run_cg_res); others run two passes per iteration. Batches iterations between host
 // checks of the device stop flag; launches after the stop exit at once.
 template <class R, class Op>
 static int run_cg(MpCtx* c, const Op& op, R* x, const R* b, R* r, R* p0, R* p1, int maxiter, int tolmode, float tol,
                   int true_every, int* iters_out, double* res_out, int kt_stencil) {
     int n = c->G.n;
+    if constexpr (!op_general<Op>::value) {
+        bool taken = false;
+        bool whole = true_every <= 0;
+        if constexpr (std::is_same<Op, PressOp>::value) whole = whole && op.rec.f != 0.0f;
+        if (whole) {
+            const int rc = run_cg_res<R, Op>(c, op, x, b, maxiter, tolmode, tol, iters_out, res_out, kt_stencil, &taken);
+            if (taken) return rc;
+        }
+    }
     int nb = c->red_blocks;
     Red Rd = red_of(c);
     cudaStream_t s = c->stream;
