@@ -88,7 +88,7 @@ struct MpCtx {
     uint32_t *keys = 0, *perm = 0;
     uint32_t *cell_cnt = 0, *cell_off = 0;   // sized for the 2x marching-cubes grid
     uint8_t *tmask = 0;
-    uint32_t *air_brick = 0;     // bit per 4x4x4-cell brick holding an AIR/AIRSOLO particle (last sort)
+    uint32_t *air_brick = 0;     // bit per brick (4^3 cells, 8^3 of the 2x grid) holding an AIR/AIRSOLO particle (last sort)
     size_t air_brick_words = 0;
     uint32_t *scan_tmp = 0;
     size_t scan_tmp_elems = 0;

@@ -17,6 +17,7 @@
 // weights already cleared, so only the lambda half-step has an effect; that is
 // what is computed here.
 #include "ctx.cuh"
+#include <type_traits>
 
 using namespace mpk;
 
@@ -28,166 +29,215 @@ struct McGrid {
     float hm;               // node spacing
 };
 
-// One thread computes NJ x NK nodes, (i, j0 + nj, k0 + nk). Neighbouring
-// nodes share most of their 4 x 4 x 4 cell windows, so the thread walks the
-// union window once, (a, b, c) ascending, and each node takes only the cells
-// of its own window: every node sees its cells, and the particles in them, in
-// the reference's (di, dj, dk, particle) order, and keeps its own per-cell
-// partial sum (res) and running sums, so each field value is bit-identical to
-// the one-node-per-thread gather. A cell's header (type mask, range) and its
-// particles are loaded once for all the nodes that need them.
-// GAS2 (with SURF == MP_MC_FLUID): the gas field is accumulated in the same
-// pass into dens2. Both surfaces use the same radius and weight, the gas
-// particles are a subset of the fluid ones, and each sum keeps its own
-// accumulators in the same visiting order, so both fields equal the separate
-// passes bit for bit.
-template <int SURF, bool GAS2, int NJ, int NK, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_mc_density(McGrid m, Tiles T, Cells cl, const float4* __restrict__ pos,
-                                                          float* __restrict__ dens, int scene, float* __restrict__ dens2) {
-    const float hm = m.hm;
-    const uint32_t need = SURF == MP_MC_SOLID ? (1u << MP_TYPESOLID)
-                        : SURF == MP_MC_FLUID ? ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO) | (1u << MP_TYPEFLUID))
-                                              : ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO));
-    const float R = SURF == MP_MC_SOLID ? hm : hm * 2;
-    const float cut = SURF == MP_MC_SOLID ? hm * hm * 1.001f : R * R * 1.001f;
+// The solid field: one thread per node, its 4 x 4 x 4 cells in the reference's
+// (di, dj, dk, particle) order with per-cell partial sums.
+__global__ void __launch_bounds__(256, 6) k_mc_density_solid(McGrid m, Tiles T, Cells cl, const float4* __restrict__ pos,
+                                                             float* __restrict__ dens) {
+    const float hm = m.hm, R = hm;
+    const float cut = hm * hm * 1.001f;
     MP_GRID_LOOP(t, T.threads()) {
-        int i, jt, kt; if (!tile_ijk(T, t, i, jt, kt)) continue;
-        const int j0 = jt * NJ, k0 = kt * NK;
-        const float px = (float)i * hm;
-        float py[NJ], pz[NK];
-        #pragma unroll
-        for (int n = 0; n < NJ; n++) py[n] = (float)(j0 + n) * hm;
-        #pragma unroll
-        for (int n = 0; n < NK; n++) pz[n] = (float)(k0 + n) * hm;
-        float cx[NJ][NK], cy[NJ][NK], cz[NJ][NK], ws[NJ][NK];
-        float gx[NJ][NK], gy[NJ][NK], gz[NJ][NK], gw[NJ][NK];
-        #pragma unroll
-        for (int u = 0; u < NJ; u++)
-            #pragma unroll
-            for (int v = 0; v < NK; v++) {
-                cx[u][v] = cy[u][v] = cz[u][v] = ws[u][v] = 0.0f;
-                gx[u][v] = gy[u][v] = gz[u][v] = gw[u][v] = 0.0f;
-            }
-        // the cell loops stay rolled: unrolled, they multiply the particle loop's
-        // code until the instruction cache misses dominate
+        int i, j, k; if (!tile_ijk(T, t, i, j, k)) continue;
+        const float3 p = mk3((float)i * hm, (float)j * hm, (float)k * hm);
+        float3 center = mk3(0.0f);
+        float wsum = 0.0f;
         #pragma unroll 1
-        for (int di = -2; di <= 1; ++di) {
-            int a = i + di; if (a < 0 || a > m.NXMC - 1) continue;
+        for (int a = max(i - 2, 0); a <= min(i + 1, m.NXMC - 1); ++a) {
             #pragma unroll 1
-            for (int b = j0 - 2; b <= j0 + NJ; ++b) {
-                if (b < 0 || b > m.NYMC - 1) continue;
+            for (int b = max(j - 2, 0); b <= min(j + 1, m.NYMC - 1); ++b) {
                 const int cb = a * m.NYMC * m.NZMC + b * m.NZMC;
-                const int cc0 = max(k0 - 2, 0), cc1 = min(k0 + NK, m.NZMC - 1);
-                // the column's cells are consecutive ranges: each cell's end is
-                // the next one's start. An empty cell adds +0 to every node's
-                // sums, which leaves them unchanged, so it is skipped.
-                uint32_t qlo = __ldg(cl.off + cb + cc0);
                 #pragma unroll 1
-                for (int cc = cc0; cc <= cc1; ++cc) {
-                    int c = cb + cc;
-                    const uint32_t q1 = __ldg(cl.off + c + 1);
-                    const uint32_t q0 = qlo;
-                    qlo = q1;
-                    if (q0 == q1 || !(__ldg(cl.tmask + c) & need)) continue;
-                    float rx[NJ][NK], ry[NJ][NK], rz[NJ][NK];
-                    float sx[NJ][NK], sy[NJ][NK], sz[NJ][NK];
-                    #pragma unroll
-                    for (int u = 0; u < NJ; u++)
-                        #pragma unroll
-                        for (int v = 0; v < NK; v++) rx[u][v] = ry[u][v] = rz[u][v] = sx[u][v] = sy[u][v] = sz[u][v] = 0.0f;
+                for (int cc = max(k - 2, 0); cc <= min(k + 1, m.NZMC - 1); ++cc) {
+                    if (!(__ldg(cl.tmask + cb + cc) & (1u << MP_TYPESOLID))) continue;
+                    float3 res = mk3(0.0f);
+                    const uint32_t q1 = __ldg(cl.off + cb + cc + 1);
                     #pragma unroll 1
-                    for (uint32_t q = q0; q < q1; ++q) {
-                        float4 o = __ldg(pos + q);
-                        int f = pflag(o);
-                        bool ok = SURF == MP_MC_SOLID ? (f == MP_TYPESOLID)
-                                : SURF == MP_MC_FLUID ? (f == MP_TYPEAIR || f == MP_TYPEAIRSOLO || f == MP_TYPEFLUID)
-                                                      : (f == MP_TYPEAIR || (f == MP_TYPEAIRSOLO && scene != MP_SCENE_INTERACTION));
-                        if (!ok) continue;
-                        const bool gas = GAS2 && (f == MP_TYPEAIR || (f == MP_TYPEAIRSOLO && scene != MP_SCENE_INTERACTION));
-                        const float dx = o.x - px;
-                        #pragma unroll
-                        for (int u = 0; u < NJ; u++) {
-                            // node j0 + u takes cells j0 + u - 2 .. j0 + u + 1
-                            if (b - j0 - u < -2 || b - j0 - u > 1) continue;
-                            const float dy = o.y - py[u];
-                            const float dxy = dx * dx + dy * dy;
-                            #pragma unroll
-                            for (int v = 0; v < NK; v++) {
-                                if (cc - k0 - v < -2 || cc - k0 - v > 1) continue;
-                                const float dz = o.z - pz[v];
-                                // dot(d, d) evaluates (x*x + y*y) + z*z; beyond the kernel
-                                // radius the weight is exactly zero and the pair adds nothing:
-                                // skip it before the sqrt (exact test with margin)
-                                const float d2 = dxy + dz * dz;
-                                if (d2 > cut) continue;
-                                const float dis = sqrtf(d2);
-                                if (!(dis < R)) continue;
-                                float w;
-                                if (SURF == MP_MC_SOLID) {
-                                    w = dis / (4 * hm);
-                                    w = 1 - w * w;
-                                    w = (float)fmax((double)(w * w * w), 0.0);
-                                } else {
-                                    w = R * R - dis * dis;
-                                    w = w * w * w;
-                                }
-                                rx[u][v] += o.x * w; ry[u][v] += o.y * w; rz[u][v] += o.z * w; ws[u][v] += w;
-                                if (gas) { sx[u][v] += o.x * w; sy[u][v] += o.y * w; sz[u][v] += o.z * w; gw[u][v] += w; }
-                            }
-                        }
+                    for (uint32_t q = __ldg(cl.off + cb + cc); q < q1; ++q) {
+                        const float4 o = __ldg(pos + q);
+                        if (pflag(o) != MP_TYPESOLID) continue;
+                        const float3 d = xyz(o) - p;
+                        const float d2 = dot(d, d);
+                        // beyond the kernel radius the pair adds nothing: skip it
+                        // before the sqrt (exact test with margin)
+                        if (d2 > cut) continue;
+                        const float dis = sqrtf(d2);
+                        if (!(dis < R)) continue;
+                        float w = dis / (4 * hm);
+                        w = 1 - w * w;
+                        w = (float)fmax((double)(w * w * w), 0.0);
+                        res.x += o.x * w; res.y += o.y * w; res.z += o.z * w; wsum += w;
                     }
-                    // a node outside this cell's window kept res = +0, and center + (+0)
-                    // is center (center is never -0: it starts at +0 and sums of finite
-                    // values round to +0)
-                    #pragma unroll
-                    for (int u = 0; u < NJ; u++)
-                        #pragma unroll
-                        for (int v = 0; v < NK; v++) {
-                            cx[u][v] += rx[u][v]; cy[u][v] += ry[u][v]; cz[u][v] += rz[u][v];
-                            if (GAS2) { gx[u][v] += sx[u][v]; gy[u][v] += sy[u][v]; gz[u][v] += sz[u][v]; }
-                        }
+                    center += res;
                 }
             }
         }
-        #pragma unroll
-        for (int u = 0; u < NJ; u++)
-            #pragma unroll
-            for (int v = 0; v < NK; v++) {
-                const int j = j0 + u, k = k0 + v;
-                if (j >= m.H || k >= m.D) continue;
-                const float3 p = mk3(px, py[u], pz[v]);
-                float3 center = mk3(cx[u][v], cy[u][v], cz[u][v]);
-                const float wsum = ws[u][v];
-                bool border = (i * j * k == 0 || i == m.NXMC || j == m.NYMC || k == m.NZMC);
-                float phi;
-                if (SURF == MP_MC_SOLID) {
-                    float r = 0.75f * hm, thigh = 0.51f, tlow = 0.49f;
-                    if (wsum > 0) {
-                        center /= wsum;
-                        float Ev = fmaxf(center.x, fmaxf(center.y, center.z)) / (4 * hm);
-                        float gamma = (thigh - Ev) / (thigh - tlow);
-                        float f = (Ev < tlow) ? 1 : gamma * gamma * gamma - 3 * gamma * gamma + 3 * gamma;
-                        phi = (length(p - center) - r * f);
-                    } else phi = -r;
-                    if (border) phi = fminf(phi, -10.0f);
-                } else {
-                    float r = SURF == MP_MC_FLUID ? 0.5f * hm : 0.8f * hm;
-                    if (wsum > 0) { center /= wsum; phi = r - length(p - center); }
-                    else phi = -r;
-                    if (border) phi = -1000.0f;
-                    if (GAS2) {
-                        const float r2 = 0.8f * hm;
-                        float3 center2 = mk3(gx[u][v], gy[u][v], gz[u][v]);
-                        const float wsum2 = gw[u][v];
-                        float phi2;
-                        if (wsum2 > 0) { center2 /= wsum2; phi2 = r2 - length(p - center2); }
-                        else phi2 = -r2;
-                        if (border) phi2 = -1000.0f;
-                        dens2[(i * m.H + j) * m.D + k] = phi2;
+        const bool border = (i * j * k == 0 || i == m.NXMC || j == m.NYMC || k == m.NZMC);
+        const float r = 0.75f * hm, thigh = 0.51f, tlow = 0.49f;
+        float phi = -r;
+        if (wsum > 0) {
+            center /= wsum;
+            float Ev = fmaxf(center.x, fmaxf(center.y, center.z)) / (4 * hm);
+            float gamma = (thigh - Ev) / (thigh - tlow);
+            float f = (Ev < tlow) ? 1 : gamma * gamma * gamma - 3 * gamma * gamma + 3 * gamma;
+            phi = (length(p - center) - r * f);
+        }
+        if (border) phi = fminf(phi, -10.0f);
+        dens[(i * m.H + j) * m.D + k] = phi;
+    }
+}
+
+// The fluid and gas fields (weight (R^2 - dis^2)^3 within R = 2 node spacings).
+// A thread computes the nodes (i, j0, k) and (i, j0 + 1, k). For each of the 4 x
+// 5 cell columns of their union window it walks the particles of the column's
+// cells k-2 .. k+1 in one loop: they are consecutive in the sorted order, and
+// with about one particle per 2x cell a loop per cell spends more on its header
+// than on its particle. Each node keeps the reference's order and sums: the
+// per-cell partial sums (res) are added to the centre when the first particle
+// of another cell comes, every node sees its cells and their particles in the
+// (di, dj, dk, particle) order, and a column outside a node's window gives it
+// weight 0. A weight is max(R^2 - dis^2, 0)^3: the rounded R^2 and dis^2 are
+// monotone in R and dis, so it is zero exactly where dis >= R, and a zero
+// weight adds +0 (the sums never hold -0). Issue-bound: about 45 instructions
+// a node and particle where the loop per cell with sqrtf took 90; warps whose
+// window touches no brick with an air particle do not carry the gas sums.
+// 256^3 fluid + gas: 37.6 -> MC_NEW ms.
+template <int SURF, bool GAS2, bool INRANGE>
+__global__ void __launch_bounds__(256, 4) k_mc_pairs(McGrid m, Tiles T, Cells cl, const float4* __restrict__ pos,
+                                                     float* __restrict__ dens, int scene, float* __restrict__ dens2,
+                                                     const uint32_t* __restrict__ air_brick) {
+    const float hm = m.hm, R = hm * 2, RR = R * R;
+    const float tiny = RR * 8.7e-19f;   // below it dis^2 does not change R^2 - dis^2
+    const uint32_t gas_types = (1u << MP_TYPEAIR) | (scene != MP_SCENE_INTERACTION ? (1u << MP_TYPEAIRSOLO) : 0u);
+    const uint32_t types = SURF == MP_MC_FLUID ? ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO) | (1u << MP_TYPEFLUID)) : gas_types;
+    // T.threads() and the stride are multiples of the warp, and a warp's lanes
+    // share i and j: all lanes take part in the votes
+    MP_GRID_LOOP(t, T.threads()) {
+        int i, jt, k;
+        const bool live = tile_ijk(T, t, i, jt, k);
+        if (!__any_sync(0xffffffffu, live)) continue;
+        const int j0 = 1 + 2 * jt;
+        i += 1; k += 1;   // the nodes inside the border
+        bool air = false;
+        if (live) {
+            const int bw = (m.NZMC + 7) / 8, bh = (m.NYMC + 7) / 8;
+            const int i0 = max(i - 2, 0) >> 3, i1 = min(i + 1, m.NXMC - 1) >> 3;
+            const int b0 = max(j0 - 2, 0) >> 3, b1 = min(j0 + 2, m.NYMC - 1) >> 3;
+            const int k0 = max(k - 2, 0) >> 3, k1 = min(k + 1, m.NZMC - 1) >> 3;
+            for (int a = i0; a <= i1; a++)
+                for (int b = b0; b <= b1; b++)
+                    for (int c = k0; c <= k1; c++) {
+                        const int br = (a * bh + b) * bw + c;
+                        air |= (__ldg(air_brick + (br >> 5)) >> (br & 31)) & 1u;
                     }
+        }
+        const bool warp_air = __any_sync(0xffffffffu, air);
+        const float px = (float)i * hm, py0 = (float)j0 * hm, py1 = (float)(j0 + 1) * hm, pz = (float)k * hm;
+        // the cells k-2 .. k+1 inside the grid, as bounds of the off entries
+        const int kb0 = live ? max(k - 2, 0) : 0, kb1 = live ? k - 1 : 0, kb2 = live ? k : 0, kb3 = live ? k + 1 : 0,
+                  kb4 = live ? min(k + 2, m.NZMC) : 0;
+        // [0..2] centre, [3..5] partial sums of the current cell; ws: weights
+        float c0[6] = {0, 0, 0, 0, 0, 0}, c1[6] = {0, 0, 0, 0, 0, 0}, ws0 = 0, ws1 = 0;
+        float g0[6] = {0, 0, 0, 0, 0, 0}, g1[6] = {0, 0, 0, 0, 0, 0}, gw0 = 0, gw1 = 0;
+        auto add = [](float (&c)[6], float& ws, float keep, float flush, float ox, float oy, float oz, float w) {
+            // centre += res when another cell starts (x * 1 + y and x * 0 + y
+            // are exact, one rounding each as the plain sums)
+            c[0] = __fmaf_rn(c[3], flush, c[0]); c[1] = __fmaf_rn(c[4], flush, c[1]); c[2] = __fmaf_rn(c[5], flush, c[2]);
+            c[3] = __fmaf_rn(c[3], keep, ox * w); c[4] = __fmaf_rn(c[4], keep, oy * w); c[5] = __fmaf_rn(c[5], keep, oz * w);
+            ws += w;
+        };
+        auto close = [](float (&c)[6]) {
+            #pragma unroll
+            for (int e = 0; e < 3; e++) { c[e] += c[e + 3]; c[e + 3] = 0.0f; }
+        };
+        auto walk = [&](auto u0, auto u1, auto with_gas, int cb) {
+            constexpr bool U0 = decltype(u0)::value, U1 = decltype(u1)::value, GAS = decltype(with_gas)::value;
+            const uint32_t* o = cl.off + cb;
+            const uint32_t B0 = __ldg(o + kb0), B1 = __ldg(o + kb1), B2 = __ldg(o + kb2), B3 = __ldg(o + kb3), B4 = __ldg(o + kb4);
+            #pragma unroll 1
+            for (uint32_t q = B0; q < B4; ++q) {
+                const float4 s = __ldg(pos + q);
+                const uint32_t f = (uint32_t)pflag(s);
+                const float dx = s.x - px, dz = s.z - pz;
+                const float xx = dx * dx, zz = dz * dz;
+                const float dy0 = s.y - py0, dy1 = s.y - py1;
+                const float e0 = (xx + dy0 * dy0) + zz, e1 = (xx + dy1 * dy1) + zz;
+                const bool first = q == B0 || q == B1 || q == B2 || q == B3;
+                // other types, and positions that are not finite, add nothing
+                if (!(((types >> (f & 31u)) & 1u) && (U0 ? e0 : e1) < 1e30f)) {
+                    if (first) {
+                        if (U0) { close(c0); if (GAS) close(g0); }
+                        if (U1) { close(c1); if (GAS) close(g1); }
+                    }
+                    continue;
                 }
-                dens[(i * m.H + j) * m.D + k] = phi;
+                const float flush = first ? 1.0f : 0.0f, keep = 1.0f - flush;
+                auto weight = [&](float d2) {
+                    const float dc = fmaxf(d2, tiny);
+                    const float dis = INRANGE ? sqrt_in_range(dc) : sqrtf(dc);
+                    const float w = fmaxf(RR - dis * dis, 0.0f);
+                    return w * w * w;
+                };
+                const bool gas = GAS && ((gas_types >> (f & 31u)) & 1u);
+                if (U0) {
+                    const float w = weight(e0);
+                    add(c0, ws0, keep, flush, s.x, s.y, s.z, w);
+                    if (GAS) add(g0, gw0, keep, flush, s.x, s.y, s.z, gas ? w : 0.0f);
+                }
+                if (U1) {
+                    const float w = weight(e1);
+                    add(c1, ws1, keep, flush, s.x, s.y, s.z, w);
+                    if (GAS) add(g1, gw1, keep, flush, s.x, s.y, s.z, gas ? w : 0.0f);
+                }
             }
+        };
+        // a column with its gas sums only where a lane's cells in it hold an air
+        // particle: most warps near a bubble meet it in a few columns
+        auto column = [&](auto u0, auto u1, int cb) {
+            if (GAS2 && warp_air) {
+                bool here = false;
+                const uint8_t* tm = cl.tmask + cb;
+                for (int c = kb0; c < kb4; c++) here |= (__ldg(tm + c) & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO))) != 0;
+                if (__any_sync(0xffffffffu, here)) { walk(u0, u1, std::true_type{}, cb); return; }
+            }
+            walk(u0, u1, std::false_type{}, cb);
+        };
+        if (SURF == MP_MC_FLUID || warp_air) {
+            using T1 = std::true_type; using F1 = std::false_type;
+            #pragma unroll 1
+            for (int a = max(i - 2, 0); a <= min(i + 1, m.NXMC - 1); ++a) {
+                const int col = a * m.NYMC * m.NZMC + (j0 - 2) * m.NZMC;
+                if (j0 - 2 >= 0) column(T1{}, F1{}, col);
+                #pragma unroll 1
+                for (int b = j0 - 1; b <= min(j0 + 1, m.NYMC - 1); ++b) column(T1{}, T1{}, col + (b - j0 + 2) * m.NZMC);
+                if (j0 + 2 < m.NYMC) column(F1{}, T1{}, col + 4 * m.NZMC);
+            }
+        }
+        if (!live) continue;
+        #pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int j = j0 + u;
+            if (j > m.H - 2) continue;
+            const float3 p = mk3(px, u ? py1 : py0, pz);
+            auto field = [&](const float (&c)[6], float ws, float r) {
+                if (!(ws > 0)) return -r;
+                return r - length(p - mk3(c[0] + c[3], c[1] + c[4], c[2] + c[5]) / ws);
+            };
+            const int idx = (i * m.H + j) * m.D + k;
+            dens[idx] = field(u ? c1 : c0, u ? ws1 : ws0, SURF == MP_MC_FLUID ? 0.5f * hm : 0.8f * hm);
+            if (GAS2) dens2[idx] = field(u ? g1 : g0, u ? gw1 : gw0, 0.8f * hm);
+        }
+    }
+}
+// the border nodes of one or two fields
+__global__ void k_mc_border(McGrid m, float* __restrict__ dens, float* __restrict__ dens2) {
+    const int fi = m.H * m.D, fj = m.W * m.D, fk = m.W * m.H;
+    MP_GRID_LOOP(t, 2 * (fi + fj + fk)) {
+        int r = t, i, j, k;
+        if (r < 2 * fi) { i = r < fi ? 0 : m.W - 1; r %= fi; j = r / m.D; k = r % m.D; }
+        else if ((r -= 2 * fi) < 2 * fj) { j = r < fj ? 0 : m.H - 1; r %= fj; i = r / m.D; k = r % m.D; }
+        else { r -= 2 * fj; k = r < fk ? 0 : m.D - 1; r %= fk; i = r / m.H; j = r % m.H; }
+        const int idx = (i * m.H + j) * m.D + k;
+        dens[idx] = -1000.0f;
+        if (dens2) dens2[idx] = -1000.0f;
     }
 }
 
@@ -352,33 +402,24 @@ static McGrid mc_grid(const MpCtx* c) {
     return m;
 }
 
-// nodes per thread of the density gather (along j, along k) and its
-// resident-blocks hint, for the single-field and the fused fluid + gas passes
-#ifndef MC_DENS_NJ
-#define MC_DENS_NJ 1
-#endif
-#ifndef MC_DENS_NK
-#define MC_DENS_NK 1
-#endif
-#ifndef MC_DENS_MINB
-#define MC_DENS_MINB 6
-#endif
-#ifndef MC_GAS2_NJ
-#define MC_GAS2_NJ 2
-#endif
-#ifndef MC_GAS2_NK
-#define MC_GAS2_NK 1
-#endif
-#ifndef MC_GAS2_MINB
-#define MC_GAS2_MINB 4
-#endif
+// the density gather of one surface, or of fluid and gas together (dens2)
 template <int SURF, bool GAS2>
-static void launch_density(const McGrid& m, Cells cl, const float4* pos, float* dens, int scene, float* dens2,
-                           cudaStream_t s) {
-    constexpr int NJ = GAS2 ? MC_GAS2_NJ : MC_DENS_NJ, NK = GAS2 ? MC_GAS2_NK : MC_DENS_NK;
-    constexpr int MINB = GAS2 ? MC_GAS2_MINB : MC_DENS_MINB;
-    const Tiles T = make_tiles(m.W, (m.H + NJ - 1) / NJ, (m.D + NK - 1) / NK);
-    k_mc_density<SURF, GAS2, NJ, NK, MINB><<<mp_blocks(T.threads(), 256), 256, 0, s>>>(m, T, cl, pos, dens, scene, dens2);
+static void launch_density(MpCtx* c, const McGrid& m, float* dens, float* dens2) {
+    const Cells cl{c->cell_off, c->tmask};
+    if constexpr (SURF == MP_MC_SOLID) {
+        const Tiles T = make_tiles(m.W, m.H, m.D);
+        k_mc_density_solid<<<mp_blocks(T.threads(), 256), 256, 0, c->stream>>>(m, T, cl, c->pos, dens);
+    } else {
+        const Tiles T = make_tiles(m.W - 2, (m.H - 1) / 2, m.D - 2);   // two interior nodes along j per thread
+        // node spacings whose squares, and those times 2^-60, are well inside
+        // the range of sqrt_in_range; other scales take sqrtf
+        const bool in_range = m.hm > 1e-5f && m.hm < 1e10f;
+        auto k = in_range ? k_mc_pairs<SURF, GAS2, true> : k_mc_pairs<SURF, GAS2, false>;
+        k<<<mp_blocks(T.threads(), 256), 256, 0, c->stream>>>(m, T, cl, c->pos, dens, c->P.scene, dens2, c->air_brick);
+        const long long edge = 2LL * (m.H * m.D + m.W * m.D + m.W * m.H);
+        k_mc_border<<<mp_blocks(edge, 256), 256, 0, c->stream>>>(m, dens, dens2);
+        c->launches++;
+    }
 }
 static int mc_extract(MpCtx* c, const McGrid& m, int surface, const float* dens);
 
@@ -386,7 +427,6 @@ static int mc_extract(MpCtx* c, const McGrid& m, int surface, const float* dens)
 int k_mc(MpCtx* c, int surface) {
     if (!c->mc_sorted) { c->err = "mc: particles are not sorted on the 2x grid (call mp_mc_presort)"; return MP_ERR_STATE; }
     const McGrid m = mc_grid(c);
-    Cells cl{c->cell_off, c->tmask};
     cudaStream_t s = c->stream;
     bool solid_empty = false;
     if (surface == MP_MC_SOLID) {
@@ -403,9 +443,9 @@ int k_mc(MpCtx* c, int surface) {
         k_mc_solid_empty<<<mp_blocks((long long)m.W * m.H * m.D, 256), 256, 0, s>>>(m, c->mc_dens);
     } else {
         KtScope kt(c, MP_KT_MC_DENS);
-        if (surface == MP_MC_SOLID) launch_density<MP_MC_SOLID, false>(m, cl, c->pos, c->mc_dens, c->P.scene, nullptr, s);
-        else if (surface == MP_MC_FLUID) launch_density<MP_MC_FLUID, false>(m, cl, c->pos, c->mc_dens, c->P.scene, nullptr, s);
-        else launch_density<MP_MC_GAS, false>(m, cl, c->pos, c->mc_dens, c->P.scene, nullptr, s);
+        if (surface == MP_MC_SOLID) launch_density<MP_MC_SOLID, false>(c, m, c->mc_dens, nullptr);
+        else if (surface == MP_MC_FLUID) launch_density<MP_MC_FLUID, false>(c, m, c->mc_dens, nullptr);
+        else launch_density<MP_MC_GAS, false>(c, m, c->mc_dens, nullptr);
     }
     c->launches++;
     return mc_extract(c, m, surface, c->mc_dens);
@@ -416,10 +456,9 @@ int k_mc(MpCtx* c, int surface) {
 int k_mc_fluid_gas(MpCtx* c) {
     if (!c->mc_sorted) { c->err = "mc: particles are not sorted on the 2x grid (call mp_mc_presort)"; return MP_ERR_STATE; }
     const McGrid m = mc_grid(c);
-    Cells cl{c->cell_off, c->tmask};
     {
         KtScope kt(c, MP_KT_MC_DENS);
-        launch_density<MP_MC_FLUID, true>(m, cl, c->pos, c->mc_dens, c->P.scene, c->mc_dens2, c->stream);
+        launch_density<MP_MC_FLUID, true>(c, m, c->mc_dens, c->mc_dens2);
     }
     c->launches++;
     MP_TRY(mc_extract(c, m, MP_MC_FLUID, c->mc_dens));

@@ -221,21 +221,21 @@ __global__ void k_segsort(const uint32_t* __restrict__ off, int ncell, uint32_t*
     }
 }
 // each cell's type mask (which particle types it holds) from the particles'
-// type bytes in cell order (coalesced reads), and with `air_words` (the
-// simulation grid's sort) the bit of each 4x4x4-cell brick that holds an AIR
-// or AIRSOLO particle
+// type bytes in cell order (coalesced reads), and the bit of each brick (4^3
+// cells of the simulation grid, 8^3 of the 2x grid: bs = 2 or 3, as many bricks
+// on both) that holds an AIR or AIRSOLO particle
 __global__ void k_tmask_sorted(const uint32_t* __restrict__ off, int ncell, int w, int hh, int d,
                                const uint8_t* __restrict__ types, uint8_t* __restrict__ tmask,
-                               uint32_t* __restrict__ air_words) {
+                               uint32_t* __restrict__ air_words, int bs) {
     MP_GRID_LOOP(cc, ncell) {
         uint32_t m = 0;
         for (uint32_t s = off[cc]; s < off[cc + 1]; s++) m |= 1u << __ldg(types + s);
         tmask[cc] = (uint8_t)m;
-        if (air_words && (m & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO)))) {
+        if ((m & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO)))) {
             const uint32_t kk = (uint32_t)cc % (uint32_t)d, jj = ((uint32_t)cc / (uint32_t)d) % (uint32_t)hh,
                            ii = (uint32_t)cc / ((uint32_t)d * (uint32_t)hh);
-            const uint32_t bw = ((uint32_t)d + 3) / 4, bh = ((uint32_t)hh + 3) / 4;
-            const uint32_t br = ((ii >> 2) * bh + (jj >> 2)) * bw + (kk >> 2);
+            const uint32_t up = (1u << bs) - 1, bw = ((uint32_t)d + up) >> bs, bh = ((uint32_t)hh + up) >> bs;
+            const uint32_t br = ((ii >> bs) * bh + (jj >> bs)) * bw + (kk >> bs);
             atomicOr(air_words + (br >> 5), 1u << (br & 31));
         }
     }
@@ -260,10 +260,10 @@ static int sort_on_grid(MpCtx* c, float dx, int w, int hh, int d) {
     uint32_t* unsorted = c->u32_scratch + 1;
     MP_CUDA(c, cudaMemsetAsync(unsorted, 0, sizeof(uint32_t), c->stream));
     const bool sim_grid = w == c->G.NX && hh == c->G.NY && d == c->G.NZ;
-    if (sim_grid) MP_CUDA(c, cudaMemsetAsync(c->air_brick, 0, sizeof(uint32_t) * c->air_brick_words, c->stream));
+    MP_CUDA(c, cudaMemsetAsync(c->air_brick, 0, sizeof(uint32_t) * c->air_brick_words, c->stream));
     auto tmask_pass = [&](const uint8_t* types) -> int {
         k_tmask_sorted<<<mp_blocks(ncell, 256), 256, 0, c->stream>>>(c->cell_off, ncell, w, hh, d, types, c->tmask,
-                                                                     sim_grid ? c->air_brick : nullptr);
+                                                                     c->air_brick, sim_grid ? 2 : 3);
         c->launches++;
         MP_CHECK_LAUNCH(c);
         return MP_OK;
