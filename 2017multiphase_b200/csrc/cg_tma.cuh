@@ -4,20 +4,30 @@
 // the scalar slots).
 //
 // One CTA owns a tile of TJ x TK cells in the (j, k) plane and marches along i
-// over a chunk of planes. For every plane q the ring holds, as TMA boxes of
-// the plane:
-//   MODE 0 (direction): r and p_old with a one-cell halo in j and k
+// over a chunk of planes, one thread per float4 group. Step t of the march
+// brings, as TMA boxes into a ring of stages,
+//   MODE 0 (direction): r and p_old of plane t with a one-cell halo in j and k
 //                       (the box starts 4 floats before the tile so that its
 //                       x coordinate stays 16-byte aligned), and the
-//                       neighbour bytes of the tile;
-//   MODE 1 (update):    p with the same halo, x, r and the neighbour bytes.
-// The CTA turns the box into the plane's stencil operand once, in a window of
-// four planes (MODE 0: p = r + beta p_old, the direction vector, computed once
-// per cell instead of once per stencil tap; MODE 1: p copied), and applies the
-// 7-point row of plane q-1 from the window planes q-2, q-1, q. The operands
-// and their arithmetic order are those of k_cg_v4 (PressOp/HeatOp::apply), so
-// the vectors it writes are the same bit for bit; only the FP64 dot product
-// adds its terms in another order. Loads run NS-1 planes ahead of the stencil.
+//                       neighbour bytes of plane t-1;
+//   MODE 1 (update):    p of plane t with the same halo; x, r and the
+//                       neighbour bytes of plane t-1;
+// and applies the 7-point row of plane t-1. A thread keeps its own group of
+// planes t-2, t-1 and t in registers (the +-i neighbours and the centre); the
+// +-j and +-k neighbours of plane t-1 come from shared memory: in MODE 0 from a
+// window of three planes of p = r + beta p_old, formed once per cell (the 64
+// halo groups by the first two warps), in MODE 1 from the ring itself.
+// Both passes were bound by issue (66 % active, 61 instructions a cell): the
+// selects for walls, the copy of every plane through a window and the FP64
+// products, which are now one fused operation (the product of two floats is
+// exact). A warp takes the selects along i and j only where one of its cells has
+// such a wall, those along k only at the ends of rows.
+// MODE 0 marches up and MODE 1 down: the planes that a pass touches last are
+// the first that the next one reads, from L2 (126 MB of the 13 bytes a cell that
+// both passes read) instead of HBM.
+// The operands and their arithmetic order are those of k_cg_v4
+// (PressOp/HeatOp::apply), so the vectors it writes are the same bit for bit;
+// only the FP64 dot product adds its terms in another order.
 //
 // Requirements checked by the host: FP32 vectors, NZ a multiple of 16 (the
 // neighbour-byte box's row stride), every vector 16-byte aligned. The tensor
@@ -28,45 +38,30 @@
 
 namespace {
 
-#ifndef TT_NS0
-#define TT_NS0 3
-#endif
-#ifndef TT_CTAS0
-#define TT_CTAS0 4
-#endif
-#ifndef TT_NS1
-#define TT_NS1 2
-#endif
-#ifndef TT_CTAS1
-#define TT_CTAS1 4
-#endif
 constexpr int TT_K = 64;              // tile cells along k (16 float4 groups)
 constexpr int TT_J = 16;              // tile rows along j
 constexpr int TT_THREADS = TT_J * (TT_K / 4);   // one thread per float4 group: 256
 constexpr int TT_HK = TT_K + 8;       // halo box along k: k0-4 .. k0+TK+3 (72 floats)
 constexpr int TT_HJ = TT_J + 2;       // halo box along j: j0-1 .. j0+TJ (18 rows)
-// ring stages and resident CTAs per SM. Both passes are bound by issue
-// latency at the occupancy shared memory allows, so more resident warps beat
-// deeper prefetch: the direction pass keeps two planes in flight with 4 CTAs
-// of 54 KB per SM (faster than three planes with 3 CTAs of 65 KB, and than
-// one plane with 5 CTAs of 43 KB); the update pass, whose stages are larger,
-// keeps one plane in flight with 4 CTAs of 49 KB (faster than two planes with
-// 3 CTAs of 63 KB)
-template <int MODE> __host__ __device__ constexpr int tt_ns() { return MODE == 0 ? TT_NS0 : TT_NS1; }
-template <int MODE> __host__ __device__ constexpr int tt_ctas() { return MODE == 0 ? TT_CTAS0 : TT_CTAS1; }
-constexpr int TT_NW = 4;              // window planes
+// stages in flight and resident CTAs per SM: both passes keep two planes in
+// flight at 4 CTAs per SM
+constexpr int TT_CTAS = 4;
+constexpr int TT_D = 2;               // steps loaded ahead
 constexpr uint32_t TT_HALO_BYTES = TT_HK * TT_HJ * 4;        // 5184
 constexpr uint32_t TT_HALO_PAD = (TT_HALO_BYTES + 127) / 128 * 128;   // 5248
 constexpr uint32_t TT_TILE_BYTES = TT_K * TT_J * 4;          // 4096
 constexpr uint32_t TT_NB_BYTES = TT_K * TT_J;                // 1024
-// stage layout (byte offsets, each 128-byte aligned)
-//   MODE 0: [halo r][halo p_old][nb]        MODE 1: [halo p][x][r][nb]
-constexpr uint32_t TT_STAGE0 = 2 * TT_HALO_PAD + TT_NB_BYTES;
-constexpr uint32_t TT_STAGE1 = TT_HALO_PAD + 2 * TT_TILE_BYTES + TT_NB_BYTES;
-constexpr uint32_t TT_WIN_BYTES = TT_NW * TT_HALO_BYTES;
-template <int MODE> __host__ __device__ constexpr uint32_t tt_stage_bytes() { return MODE == 0 ? TT_STAGE0 : TT_STAGE1; }
+// MODE 0: TT_D + 1 stages [halo r][halo p_old][nb], then a 3-plane window of p
+// MODE 1: TT_D + 1 stages [x][r][nb], then TT_D + 2 planes [halo p]
+// (each part 128-byte aligned)
+constexpr int TT_NS = TT_D + 1;
+template <int MODE> __host__ __device__ constexpr uint32_t tt_stage_bytes() {
+    return MODE == 0 ? 2 * TT_HALO_PAD + TT_NB_BYTES : 2 * TT_TILE_BYTES + TT_NB_BYTES;
+}
+constexpr int TT_NP = TT_D + 2;       // MODE 1's planes of p: t-1 and t are read, TT_D are in flight
+constexpr int TT_NW = 3;              // MODE 0's window: t-1 read while t is written, and t+1 by a faster warp
 template <int MODE> __host__ __device__ constexpr uint32_t tt_smem_bytes() {
-    return tt_ns<MODE>() * tt_stage_bytes<MODE>() + TT_WIN_BYTES + tt_ns<MODE>() * 8 + 128;   // + barriers, alignment
+    return TT_NS * tt_stage_bytes<MODE>() + (MODE == 0 ? TT_NW : TT_NP) * TT_HALO_PAD + TT_NS * 8 + 128;   // + barriers, alignment
 }
 // a wait on a TMA barrier gives up after this long (ns) and reports MP_ERR_TIMEOUT
 constexpr unsigned long long TT_WAIT_NS = 1000000000ull;
@@ -178,7 +173,7 @@ struct TtMaps {
 // MODE 0: p_new = r + beta p_old (first: r); z = A p_new; p_new . z
 // MODE 1: z = A p; x += alpha p, r -= alpha z; r . r; stop test
 template <class Op, int MODE>
-__global__ void __launch_bounds__(TT_THREADS, tt_ctas<MODE>())
+__global__ void __launch_bounds__(TT_THREADS, TT_CTAS)
     k_cg_tma(Op op, const __grid_constant__ TtMaps maps, float* __restrict__ pout, float* __restrict__ x,
              float* __restrict__ r, Red Rd, int chunk, int first, int it, int maxiter, int skip_dot) {
     // launched with programmatic stream serialization: the previous launch on
@@ -189,9 +184,8 @@ __global__ void __launch_bounds__(TT_THREADS, tt_ctas<MODE>())
     extern __shared__ unsigned char tt_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tt_raw) + 127) & ~uintptr_t(127));
     constexpr uint32_t SB = tt_stage_bytes<MODE>();
-    constexpr int TT_NS = tt_ns<MODE>();
-    float* win = reinterpret_cast<float*>(sm + TT_NS * SB);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + TT_NS * SB + TT_WIN_BYTES);
+    unsigned char* planes = sm + TT_NS * SB;   // window of p (MODE 0) or ring of p (MODE 1)
+    uint64_t* bar = reinterpret_cast<uint64_t*>(planes + (MODE == 0 ? TT_NW : TT_NP) * TT_HALO_PAD);
     __shared__ int tt_fail;
 
     const Grid& g = op.g;
@@ -203,126 +197,138 @@ __global__ void __launch_bounds__(TT_THREADS, tt_ctas<MODE>())
     const bool inb = kk < g.NZ && jj < g.NY;
     const float bf = (MODE == 0 && !first) ? (float)Rd.scal[S_BETA] : 0.0f;
     const float af = MODE == 1 ? (float)Rd.scal[S_ALPHA] : 0.0f;
-    const bool load_b = MODE == 1 || !first;
-    const uint32_t tx = MODE == 0 ? (load_b ? 2 * TT_HALO_BYTES : TT_HALO_BYTES) + TT_NB_BYTES
-                                  : TT_HALO_BYTES + 2 * TT_TILE_BYTES + TT_NB_BYTES;
-    // planes q = i0-1 .. i1 pass through the ring; plane q uses stage (q - i0 + 1) % NS
-    const int q0 = i0 - 1, nplanes = i1 - i0 + 2;
-
-    auto issue = [&](int t) {   // plane q0 + t into stage t % NS (thread 0)
+    const bool load_b = MODE == 0 && !first;
+    // steps t = 0 .. nsteps-1 pass planes i0-1 .. i1 (MODE 0) or i1 .. i0-1 (MODE 1)
+    const int nsteps = i1 - i0 + 2;
+    auto plane_of = [&](int t) { return MODE == 0 ? i0 - 1 + t : i1 - t; };
+    auto issue = [&](int t) {   // thread 0
         unsigned char* st = sm + (t % TT_NS) * SB;
         uint64_t* b = bar + (t % TT_NS);
-        const int q = q0 + t;
-        tt_bar_expect(b, tx);
+        const int q = plane_of(t), qc = plane_of(t - 1);
+        const bool row = t >= 2;   // plane t-1 is one of the chunk's: its row is formed in step t
         if (MODE == 0) {
+            tt_bar_expect(b, (load_b ? 2 * TT_HALO_BYTES : TT_HALO_BYTES) + (row ? TT_NB_BYTES : 0));
             tt_load(st, &maps.a, b, k0 - 4, j0 - 1, q);
             if (load_b) tt_load(st + TT_HALO_PAD, &maps.b, b, k0 - 4, j0 - 1, q);
-            tt_load(st + 2 * TT_HALO_PAD, &maps.nb, b, k0, j0, q);
+            if (row) tt_load(st + 2 * TT_HALO_PAD, &maps.nb, b, k0, j0, qc);
         } else {
-            tt_load(st, &maps.a, b, k0 - 4, j0 - 1, q);
-            tt_load(st + TT_HALO_PAD, &maps.b, b, k0, j0, q);
-            tt_load(st + TT_HALO_PAD + TT_TILE_BYTES, &maps.c, b, k0, j0, q);
-            tt_load(st + TT_HALO_PAD + 2 * TT_TILE_BYTES, &maps.nb, b, k0, j0, q);
+            tt_bar_expect(b, TT_HALO_BYTES + (row ? 2 * TT_TILE_BYTES + TT_NB_BYTES : 0));
+            tt_load(planes + (t % TT_NP) * TT_HALO_PAD, &maps.a, b, k0 - 4, j0 - 1, q);
+            if (row) {
+                tt_load(st, &maps.b, b, k0, j0, qc);
+                tt_load(st + TT_TILE_BYTES, &maps.c, b, k0, j0, qc);
+                tt_load(st + 2 * TT_TILE_BYTES, &maps.nb, b, k0, j0, qc);
+            }
         }
     };
     if (tid == 0) {
         tt_fail = 0;
         for (int s = 0; s < TT_NS; s++) tt_bar_init(bar + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int t = 0; t < TT_NS && t < nplanes; t++) issue(t);
+        for (int t = 0; t < TT_D && t < nsteps; t++) issue(t);
     }
     __syncthreads();
 
+    // float4 places in a halo box of this thread's group and, for the first two
+    // warps, of a halo group: rows 0 and 17 beside the tile, columns 0 and 17
+    constexpr int HG = TT_HK / 4;
+    const int own = (ty + 1) * HG + 1 + tg;
+    const int halo = tid < 16 ? 1 + tid : (tid < 32 ? (TT_HJ - 1) * HG + 1 + (tid - 16)
+                                                    : (1 + ((tid - 32) >> 1)) * HG + (tid & 1) * (HG - 1));
     double acc = 0;
-    // this thread's group of the previous plane: neighbour bytes, x, r
-    uint32_t m_prev = 0;
-    float4 x_prev = make_float4(0, 0, 0, 0), r_prev = x_prev;
+    float4 v0 = make_float4(0, 0, 0, 0), v1 = v0;   // own group of planes t-2 and t-1
     int t = 0;
-    for (; t < nplanes; t++) {
-        const int q = q0 + t;
+    for (; t < nsteps; t++) {
         unsigned char* st = sm + (t % TT_NS) * SB;
         // every thread waits for the stage itself; a wait that runs out is
         // seen by all threads after the barrier below
         const bool ok = tt_bar_wait(bar + (t % TT_NS), (uint32_t)((t / TT_NS) & 1));
         if (!ok) atomicExch(&tt_fail, 1);
-        // the window plane of q from the stage
-        float4* w = reinterpret_cast<float4*>(win + (t % TT_NW) * (TT_HK * TT_HJ));
-        const float4* sa = reinterpret_cast<const float4*>(st);
-        const float4* sb = reinterpret_cast<const float4*>(st + TT_HALO_PAD);
-        for (int e = tid; ok && e < TT_HK * TT_HJ / 4; e += TT_THREADS) {
-            float4 a = sa[e];
-            if (MODE == 0 && !first) {
-                const float4 b = sb[e];
-                a = make_float4(a.x + bf * b.x, a.y + bf * b.y, a.z + bf * b.z, a.w + bf * b.w);
-            }
-            w[e] = a;
-        }
-        // this thread's own group of plane q
-        uint32_t m_cur;
-        float4 x_cur = make_float4(0, 0, 0, 0), r_cur = x_cur;
+        float4 v2;                                    // own group of plane t
+        float4* wt = reinterpret_cast<float4*>(planes + (t % (MODE == 0 ? TT_NW : TT_NP)) * TT_HALO_PAD);
         if (MODE == 0) {
-            m_cur = reinterpret_cast<const uint32_t*>(st + 2 * TT_HALO_PAD)[tid];
+            const float4* sa = reinterpret_cast<const float4*>(st);
+            const float4* sb = reinterpret_cast<const float4*>(st + TT_HALO_PAD);
+            auto form = [&](int e) {
+                float4 a = sa[e];
+                if (!first) {
+                    const float4 b = sb[e];
+                    a = make_float4(a.x + bf * b.x, a.y + bf * b.y, a.z + bf * b.z, a.w + bf * b.w);
+                }
+                wt[e] = a;
+                return a;
+            };
+            v2 = form(own);
+            if (tid < 64) form(halo);
         } else {
-            x_cur = reinterpret_cast<const float4*>(st + TT_HALO_PAD)[tid];
-            r_cur = reinterpret_cast<const float4*>(st + TT_HALO_PAD + TT_TILE_BYTES)[tid];
-            m_cur = reinterpret_cast<const uint32_t*>(st + TT_HALO_PAD + 2 * TT_TILE_BYTES)[tid];
+            v2 = wt[own];
         }
-        // every thread has read stage t: order those reads before the TMA
-        // writes that refill it, and publish the window plane
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // all threads are past step t-1, whose stage (and, MODE 1, plane t-2 of
+        // the ring) is free, and have read stage t's r and p_old (MODE 0)
         __syncthreads();
         if (tt_fail) break;
-        if (tid == 0 && t + TT_NS < nplanes) issue(t + TT_NS);
-        // the row of plane q-1 from window planes q-2, q-1, q
-        const int ic = q - 1;
-        if (t >= 2 && inb && (m_prev & 0x80808080u)) {
-            const float* wm = win + ((t - 2) % TT_NW) * (TT_HK * TT_HJ);
-            const float* wc = win + ((t - 1) % TT_NW) * (TT_HK * TT_HJ);
-            const float* wp = win + (t % TT_NW) * (TT_HK * TT_HJ);
-            const int o = (ty + 1) * TT_HK + 4 + 4 * tg;
-            const float4 c = *reinterpret_cast<const float4*>(wc + o);
-            const float4 xp = *reinterpret_cast<const float4*>(wp + o);
-            const float4 xm = *reinterpret_cast<const float4*>(wm + o);
-            const float4 yp = *reinterpret_cast<const float4*>(wc + o + TT_HK);
-            const float4 ym = *reinterpret_cast<const float4*>(wc + o - TT_HK);
-            const float zm = wc[o - 1], zp = wc[o + 4];
-            const float cv[6] = {zm, c.x, c.y, c.z, c.w, zp};
-            const float xpv[4] = {xp.x, xp.y, xp.z, xp.w}, xmv[4] = {xm.x, xm.y, xm.z, xm.w};
-            const float ypv[4] = {yp.x, yp.y, yp.z, yp.w}, ymv[4] = {ym.x, ym.y, ym.z, ym.w};
-            float xov[4] = {x_prev.x, x_prev.y, x_prev.z, x_prev.w}, rov[4] = {r_prev.x, r_prev.y, r_prev.z, r_prev.w};
-            float po[4];
-            const int cidx = (ic * g.NY + jj) * g.NZ + kk;
-            #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const uint32_t m = (m_prev >> (8 * e)) & 0xffu;
-                const float cur = cv[e + 1];
-                po[e] = (m & 0x80) ? cur : 0.0f;
-                if (m & 0x80) {
-                    float s = op.template start<float>(cidx + e, cur);
-                    s = op.template comb<float>(s, (m & 1) ? cur : xpv[e]);
-                    s = op.template comb<float>(s, (m & 2) ? cur : ypv[e]);
-                    s = op.template comb<float>(s, (m & 4) ? cur : cv[e + 2]);
-                    s = op.template comb<float>(s, (m & 8) ? cur : xmv[e]);
-                    s = op.template comb<float>(s, (m & 16) ? cur : ymv[e]);
-                    s = op.template comb<float>(s, (m & 32) ? cur : cv[e]);
-                    const float z = op.template finish<float>(s);
-                    if (MODE == 0) {
-                        acc += (double)z * (double)cur;
-                    } else {
-                        xov[e] = xov[e] + af * cur;
-                        rov[e] = rov[e] + (-af) * z;
-                        acc += (double)rov[e] * (double)rov[e];
+        if (tid == 0 && t + TT_D < nsteps) issue(t + TT_D);
+        if (t >= 2) {
+            const uint32_t m4 = reinterpret_cast<const uint32_t*>(st + (MODE == 0 ? 2 * TT_HALO_PAD : 2 * TT_TILE_BYTES))[tid];
+            const bool act = inb && (m4 & 0x80808080u);
+            const bool walls = __any_sync(0xffffffffu, (m4 & 0x1b1b1b1bu) != 0);
+            const bool ends = __any_sync(0xffffffffu, m4 != 0x80808080u);
+            if (act) {
+                const float4* wc4 = reinterpret_cast<const float4*>(planes + ((t - 1) % (MODE == 0 ? TT_NW : TT_NP)) * TT_HALO_PAD);
+                const float* wc = reinterpret_cast<const float*>(wc4 + own);
+                const float4 yp = wc4[own + HG], ym = wc4[own - HG];
+                const float4 xp = MODE == 0 ? v2 : v0, xm = MODE == 0 ? v0 : v2;
+                const float cv[6] = {wc[-1], v1.x, v1.y, v1.z, v1.w, wc[4]};
+                const float xpv[4] = {xp.x, xp.y, xp.z, xp.w}, xmv[4] = {xm.x, xm.y, xm.z, xm.w};
+                const float ypv[4] = {yp.x, yp.y, yp.z, yp.w}, ymv[4] = {ym.x, ym.y, ym.z, ym.w};
+                float4 x4 = make_float4(0, 0, 0, 0), r4 = x4;
+                if (MODE == 1) {
+                    x4 = reinterpret_cast<const float4*>(st)[tid];
+                    r4 = reinterpret_cast<const float4*>(st + TT_TILE_BYTES)[tid];
+                }
+                float xov[4] = {x4.x, x4.y, x4.z, x4.w}, rov[4] = {r4.x, r4.y, r4.z, r4.w}, po[4];
+                const int cidx = (plane_of(t - 1) * g.NY + jj) * g.NZ + kk;
+                // W: walls along i or j in the warp; E: not every cell of the
+                // warp is an unknown without walls along k
+                auto cells = [&](auto with_walls, auto with_ends) {
+                    constexpr bool W = decltype(with_walls)::value, E = decltype(with_ends)::value;
+                    #pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const uint32_t m = m4 >> (8 * e);
+                        const float cur = cv[e + 1];
+                        const bool unk = !E || (m & 0x80u);
+                        po[e] = unk ? cur : 0.0f;
+                        float s = op.template start<float>(cidx + e, cur);
+                        s = op.template comb<float>(s, W && (m & 1u) ? cur : xpv[e]);
+                        s = op.template comb<float>(s, W && (m & 2u) ? cur : ypv[e]);
+                        s = op.template comb<float>(s, E && (m & 4u) ? cur : cv[e + 2]);
+                        s = op.template comb<float>(s, W && (m & 8u) ? cur : xmv[e]);
+                        s = op.template comb<float>(s, W && (m & 16u) ? cur : ymv[e]);
+                        s = op.template comb<float>(s, E && (m & 32u) ? cur : cv[e]);
+                        const float z = op.template finish<float>(s);
+                        if (unk) {
+                            if (MODE == 0) {
+                                acc = __fma_rn((double)z, (double)cur, acc);
+                            } else {
+                                xov[e] = xov[e] + af * cur;
+                                rov[e] = rov[e] + (-af) * z;
+                                acc = __fma_rn((double)rov[e], (double)rov[e], acc);
+                            }
+                        }
                     }
+                };
+                if (!ends) cells(std::false_type{}, std::false_type{});
+                else if (!walls) cells(std::false_type{}, std::true_type{});
+                else cells(std::true_type{}, std::true_type{});
+                if (MODE == 0) {
+                    reinterpret_cast<float4*>(pout)[cidx >> 2] = make_float4(po[0], po[1], po[2], po[3]);
+                } else {
+                    reinterpret_cast<float4*>(x)[cidx >> 2] = make_float4(xov[0], xov[1], xov[2], xov[3]);
+                    reinterpret_cast<float4*>(r)[cidx >> 2] = make_float4(rov[0], rov[1], rov[2], rov[3]);
                 }
             }
-            if (MODE == 0) {
-                reinterpret_cast<float4*>(pout)[cidx >> 2] = make_float4(po[0], po[1], po[2], po[3]);
-            } else {
-                reinterpret_cast<float4*>(x)[cidx >> 2] = make_float4(xov[0], xov[1], xov[2], xov[3]);
-                reinterpret_cast<float4*>(r)[cidx >> 2] = make_float4(rov[0], rov[1], rov[2], rov[3]);
-            }
         }
-        m_prev = m_cur; x_prev = x_cur; r_prev = r_cur;
+        v0 = v1; v1 = v2;
     }
     // the next pass may be launched now; it waits for this grid's completion
     // before it reads anything this grid writes
@@ -332,7 +338,7 @@ __global__ void __launch_bounds__(TT_THREADS, tt_ctas<MODE>())
         // into this CTA's ring, report the timeout and leave without joining
         // the sum (the host clears the block counter before the next solve)
         if (tid == 0) {
-            for (int u = t; u < nplanes && u < t + TT_NS; u++) tt_bar_wait(bar + (u % TT_NS), (uint32_t)((u / TT_NS) & 1));
+            for (int u = t; u < nsteps && u < t + TT_D; u++) tt_bar_wait(bar + (u % TT_NS), (uint32_t)((u / TT_NS) & 1));
             Rd.flag[F_DONE] = DONE_TIMEOUT;
         }
         return;

@@ -139,7 +139,8 @@ struct PressOp {
     template <class R> __device__ __forceinline__ R comb(R s, R v) const { return s + v; }
     CgQuot rec;   // 1 / h^2 in FP32 and FP64
     template <class R> __device__ __forceinline__ R finish(R s) const {
-        if (rec.f != 0.0f) return finish_rec<R>(s);
+        if (inv_h2 != 0.0f) return s * (R)inv_h2;
+        if (rec.f != 0.0f) return cg_quot(s, rec);
         return s / ((R)g.h * (R)g.h);
     }
     // the same when rec.f != 0 is known (no division, so no call, in the kernel)
@@ -1038,8 +1039,7 @@ static int run_cg(MpCtx* c, const Op& op, R* x, const R* b, R* r, R* p0, R* p1, 
                 const int nch = std::max(1, (148 * ctas) / (tk * tj));
                 return c->cg_tma_chunk > 0 ? c->cg_tma_chunk : std::max(4, (gg.NX + nch - 1) / nch);
             };
-            tchunk0 = chunk_for(tt_ctas<0>());
-            tchunk = chunk_for(tt_ctas<1>());
+            tchunk0 = tchunk = chunk_for(TT_CTAS);
             tgrid0 = dim3(tk, tj, (gg.NX + tchunk0 - 1) / tchunk0);
             tgrid = dim3(tk, tj, (gg.NX + tchunk - 1) / tchunk);
             if ((long long)tgrid0.x * tgrid0.y * tgrid0.z > 148LL * 32 || (long long)tgrid.x * tgrid.y * tgrid.z > 148LL * 32)
