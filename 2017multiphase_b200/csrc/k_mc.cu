@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256, 6) k_mc_density_solid(McGrid m, Tiles T, 
 // weight adds +0 (the sums never hold -0). Issue-bound: about 45 instructions
 // a node and particle where the loop per cell with sqrtf took 90; warps whose
 // window touches no brick with an air particle do not carry the gas sums.
-// 256^3 fluid + gas: 37.6 -> MC_NEW ms.
+// 256^3 fluid + gas: 37.6 -> 19 ms.
 template <int SURF, bool GAS2, bool INRANGE>
 __global__ void __launch_bounds__(256, 4) k_mc_pairs(McGrid m, Tiles T, Cells cl, const float4* __restrict__ pos,
                                                      float* __restrict__ dens, int scene, float* __restrict__ dens2,

@@ -19,121 +19,76 @@ using namespace mpk;
 
 namespace {
 
-// The air P2G (mapvelp2g_k_air, spray_k.cu:2894-2937): AIR particles, window
-// -2..1 along the face normal and -2..2 across (100 cells). One thread owns the
-// x-, y- and z-face with the same (i,j,k) and walks the union of their windows
-// once; each face accumulates only the cells of its own window, in the
-// reference's (di,dj,dk,particle) order. Bubbles are sparse, so each cell's type
-// mask is tested first and only cells with an AIR particle are walked.
-// sharp_kernel(r2, 1.4) is exactly zero once r2 exceeds 1.4^2, and a zero
-// weight adds +-0 to both sums, so such pairs are skipped, and the velocity is
-// read only when some face takes the particle.
-// A face triple whose 5x5x5-cell window touches no 4x4x4-cell brick holding an
-// air particle (the bit map of the last sort) has no pair: its faces take 0,
-// as the walk would give them.
-__global__ void __launch_bounds__(256, 4) k_p2g_air(Grid g, Cells cl, const float4* __restrict__ pos,
-                                                    const float4* __restrict__ vel, float* __restrict__ ux,
-                                                    float* __restrict__ uy, float* __restrict__ uz,
-                                                    const uint32_t* __restrict__ air_brick) {
-    constexpr int R = 2;       // union window -R..R
-    constexpr int HI = 1;      // upper bound along the face normal
-    const Tiles T = make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1);
-    const float scale = 1.0f / g.h;
-    const float cut = (1.4f * 1.4f) * 1.0001f;
-    MP_GRID_LOOP(t, T.threads()) {
-        int i, j, k; if (!tile_ijk(T, t, i, j, k)) continue;
-        bool hx = (j < g.NY && k < g.NZ), hy = (i < g.NX && k < g.NZ), hz = (i < g.NX && j < g.NY);
-        float wx = 0, sx = 0, wy = 0, sy = 0, wz = 0, sz = 0;
-        bool air_near = false;
-        {
-            const int bw = (g.NZ + 3) / 4, bh = (g.NY + 3) / 4;
-            const int bi0 = max(i - R, 0) >> 2, bi1 = min(i + R, g.NX - 1) >> 2;
-            const int bj0 = max(j - R, 0) >> 2, bj1 = min(j + R, g.NY - 1) >> 2;
-            const int bk0 = max(k - R, 0) >> 2, bk1 = min(k + R, g.NZ - 1) >> 2;
-            for (int bi = bi0; bi <= bi1 && !air_near; bi++)
-                for (int bj = bj0; bj <= bj1 && !air_near; bj++)
-                    for (int bk = bk0; bk <= bk1; bk++) {
-                        const int br = (bi * bh + bj) * bw + bk;
-                        if ((__ldg(air_brick + (br >> 5)) >> (br & 31)) & 1u) { air_near = true; break; }
-                    }
-        }
-        if (!air_near) {
-            if (hx) ux[fxi(g, i, j, k)] = 0.0f;
-            if (hy) uy[fyi(g, i, j, k)] = 0.0f;
-            if (hz) uz[fzi(g, i, j, k)] = 0.0f;
-            continue;
-        }
-        const float3 gpx = mk3((float)i, (float)j + 0.5f, (float)k + 0.5f);
-        const float3 gpy = mk3((float)i + 0.5f, (float)j, (float)k + 0.5f);
-        const float3 gpz = mk3((float)i + 0.5f, (float)j + 0.5f, (float)k);
-        const int klo = max(k - R, 0), khi = min(k + R, g.NZ - 1);
-        for (int di = -R; di <= R; di++) {
-            int a = i + di; if (a < 0 || a > g.NX - 1) continue;
-            const bool ax = hx && di <= HI;
-            for (int dj = -R; dj <= R; dj++) {
-                int b = j + dj; if (b < 0 || b > g.NY - 1) continue;
-                const bool ay = hy && dj <= HI;
-                if (!(ax || ay || hz)) continue;
-                const int cb = cid(g, a, b, 0);
-                for (int cc = klo; cc <= khi; cc++) {
-                    const bool az = hz && cc - k <= HI;
-                    if (!(ax || ay || az)) continue;
-                    // the type mask is built at sort time; AIR <-> AIRSOLO flips since then
-                    // (markSoloAirParticle) keep the union bit valid
-                    if (!(__ldg(cl.tmask + cb + cc) & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO)))) continue;
-                    const uint32_t s1 = __ldg(cl.off + cb + cc + 1);
-                    for (uint32_t p = __ldg(cl.off + cb + cc); p < s1; ++p) {
-                        const float4 q = __ldg(pos + p);
-                        if (pflag(q) != MP_TYPEAIR) continue;
-                        const float3 ps = mk3(q.x, q.y, q.z) * scale;
-                        const float3 dx = ps - gpx, dy = ps - gpy, dz = ps - gpz;
-                        const float r2x = dot(dx, dx), r2y = dot(dy, dy), r2z = dot(dz, dz);
-                        const bool tx = ax && r2x <= cut, ty = ay && r2y <= cut, tz = az && r2z <= cut;
-                        if (!(tx || ty || tz)) continue;
-                        const float4 v = __ldg(vel + p);
-                        if (tx) { float w = v.w * sharp_kernel(r2x, 1.4f); wx += w; sx += w * v.x; }
-                        if (ty) { float w = v.w * sharp_kernel(r2y, 1.4f); wy += w; sy += w * v.y; }
-                        if (tz) { float w = v.w * sharp_kernel(r2z, 1.4f); wz += w; sz += w * v.z; }
-                    }
-                }
-            }
-        }
-        if (hx) ux[fxi(g, i, j, k)] = (wx > 0) ? (sx / wx) : 0.0f;
-        if (hy) uy[fyi(g, i, j, k)] = (wy > 0) ? (sy / wy) : 0.0f;
-        if (hz) uz[fzi(g, i, j, k)] = (wz > 0) ? (sz / wz) : 0.0f;
-    }
-}
-
-#ifndef P2G_CAP
-#define P2G_CAP 320
-#endif
-#ifndef P2G_SMINB
-#define P2G_SMINB 2
-#endif
+// staged particles per warp: the 34 cells of a water column hold 272 at 8 a cell
+// (a second chunk leaves most lanes idle in each); an air column is mostly short
+constexpr int P2G_CAP = 320, P2G_AIR_CAP = 192;
 // padded slot of the t-th staged particle: one spare float4 per 8, so lanes
 // whose ranges start about a cell (8 particles) apart hit different banks
 __device__ __forceinline__ uint32_t p2g_slot(uint32_t t) { return t + (t >> 3); }
 __host__ __device__ constexpr int p2g_slots(int cap) { return cap + cap / 8; }
 
-// The water P2G (mapvelp2g_k_fluidSolid, spray_k.cu:2829-2892): FLUID and
-// SOLID particles, window -1..0 along the face normal and -1..1 across (18
-// cells), with each warp's particle loads coalesced.
+// The three faces of a node (i, j, k): sums of weights and of weighted velocities
+struct FaceSums {
+    float wx = 0, sx = 0, wy = 0, sy = 0, wz = 0, sz = 0;
+};
+// Adds the staged particles [lo, hi) to a node's faces in ascending order, the
+// z-face those below hz. A face takes a pair with r2 <= its cut (negative: the
+// face does not take this column); beyond 1.4^2 the weight is exactly zero and
+// the pair adds nothing. Weights are formed for all three faces without a branch
+// (a branch per face around a division cost 86 instructions a particle where
+// this takes about 60), the sums are predicated. Particles of another type are
+// staged far away, so no cut takes them.
+__device__ __forceinline__ void p2g_walk(const float4* __restrict__ sp, const float4* __restrict__ sv, uint32_t lo,
+                                         uint32_t hi, uint32_t hz, float3 gpx, float3 gpy, float3 gpz, float cutx,
+                                         float cuty, float cutz, FaceSums& F) {
+    #pragma unroll 2
+    for (uint32_t p = lo; p < hi; ++p) {
+        const float4 q = sp[p2g_slot(p)], v = sv[p2g_slot(p)];
+        const float3 ps = mk3(q.x, q.y, q.z);
+        const float3 dx = ps - gpx, dy = ps - gpy, dz = ps - gpz;
+        const float r2x = dot(dx, dx), r2y = dot(dy, dy), r2z = dot(dz, dz);
+        auto weight = [&](float r2) {
+            return v.w * fmaxf(quot_in_range(1.4f * 1.4f, fmaxf(r2, 0.0001f)) - 1.0f, 0.0f);
+        };
+        const float ax = weight(r2x), ay = weight(r2y), az = weight(r2z);
+        if (r2x <= cutx) { F.wx += ax; F.sx += ax * v.x; }
+        if (r2y <= cuty) { F.wy += ay; F.sy += ay * v.y; }
+        if (r2z <= cutz && p < hz) { F.wz += az; F.sz += az * v.z; }
+    }
+}
+constexpr float P2G_FAR = 1e15f;   // scaled position of a staged particle that no face takes
+
+// Both P2G gathers with each warp's particle loads coalesced.
+//   AIR = false: the water P2G (mapvelp2g_k_fluidSolid, spray_k.cu:2829-2892):
+//     FLUID and SOLID particles, window -1..0 along the face normal and -1..1
+//     across (18 cells)
+//   AIR = true: the air P2G (mapvelp2g_k_air, spray_k.cu:2894-2937): AIR
+//     particles, window -2..1 along the normal and -2..2 across (100 cells)
 // A warp holds the nodes (i, j, k0 .. k0+31); for one (di, dj) its lanes'
-// windows are overlapping ranges of the cells (a, b, k0-1 .. k0+32), which are
+// windows are overlapping ranges of the cells (a, b, k0-R .. k0+31+R), which are
 // consecutive in the sorted order. The warp copies that particle range, CAP at
-// a time, into shared memory with coalesced loads (scaled position, water test,
-// velocity and mass), then each lane walks its own part of the chunk in
-// ascending order. Per-lane loads from global memory hit ~32 separate lines per
-// warp instruction and saturate L1; the staged reads do not. Every face adds
-// the same particles in the same order with the same arithmetic as
-// the one-thread-per-face-triple gather, so the fields are bit-identical.
-template <int CAP>
-__global__ void __launch_bounds__(256, P2G_SMINB) k_p2g_water(Grid g, Cells cl, const float4* __restrict__ pos,
-                                                              const float4* __restrict__ vel, float* __restrict__ ux,
-                                                              float* __restrict__ uy, float* __restrict__ uz) {
+// a time, into shared memory with coalesced loads (scaled position, velocity
+// and mass), then each lane walks its own part of the chunk in ascending order.
+// Per-lane loads from global memory hit ~32 separate lines per warp instruction
+// and saturate L1; the staged reads do not. Every face adds the same particles
+// in the same order with the same arithmetic as the one-thread-per-face-triple
+// gather, so the fields are bit-identical.
+// Air is sparse: a warp whose windows touch no 4x4x4-cell brick with an air
+// particle (the bit map of the last sort) writes 0, a column without an air
+// cell is skipped, and only the air particles of a chunk are staged (its places
+// by a running count, so a lane's part of the chunk is again a range).
+// 256^3: water 17.6 -> 10.9 ms, air 2.6 -> 2.4 ms; 32^3: water 87 -> 51 us, air 222 -> 110 us.
+template <bool AIR, int CAP>
+__global__ void __launch_bounds__(256, AIR ? 3 : 2) k_p2g_staged(Grid g, Cells cl, const float4* __restrict__ pos,
+                                                               const float4* __restrict__ vel, float* __restrict__ ux,
+                                                               float* __restrict__ uy, float* __restrict__ uz,
+                                                               const uint32_t* __restrict__ air_brick) {
+    constexpr int R = AIR ? 2 : 1;     // union window -R..R
+    constexpr int HI = AIR ? 1 : 0;    // upper bound along the face normal
     extern __shared__ float4 p2g_sm[];
+    __shared__ uint16_t before[AIR ? 8 : 1][AIR ? CAP + 2 : 1];   // air particles of the chunk before each place
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float4* sp = p2g_sm + (size_t)warp * 2 * p2g_slots(CAP);   // (x, y, z) / h and the water test
+    float4* sp = p2g_sm + (size_t)warp * 2 * p2g_slots(CAP);   // (x, y, z) / h
     float4* sv = sp + p2g_slots(CAP);                           // velocity and mass
     const Tiles T = make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1);
     const float scale = 1.0f / g.h;
@@ -145,61 +100,108 @@ __global__ void __launch_bounds__(256, P2G_SMINB) k_p2g_water(Grid g, Cells cl, 
         const bool act = tile_ijk(T, t, i, j, k);
         // i and j are the same across the warp, and lane 0 holds the lowest k
         if (!__any_sync(0xffffffffu, act)) continue;
-        bool hx = act && (j < g.NY && k < g.NZ), hy = act && (i < g.NX && k < g.NZ), hz = act && (i < g.NX && j < g.NY);
-        float wx = 0, sx = 0, wy = 0, sy = 0, wz = 0, sz = 0;
-        const float3 gpx = mk3((float)i, (float)j + 0.5f, (float)k + 0.5f);
-        const float3 gpy = mk3((float)i + 0.5f, (float)j, (float)k + 0.5f);
-        const float3 gpz = mk3((float)i + 0.5f, (float)j + 0.5f, (float)k);
-        const int klo = max(k - 1, 0), khi = min(k + 1, g.NZ - 1);
-        for (int di = -1; di <= 1; di++) {
-            int a = i + di; if (a < 0 || a > g.NX - 1) continue;
-            const bool ax = hx && di <= 0;
-            for (int dj = -1; dj <= 1; dj++) {
-                int b = j + dj; if (b < 0 || b > g.NY - 1) continue;
-                const bool ay = hy && dj <= 0;
-                const bool need = ax || ay || hz;
-                if (!__any_sync(0xffffffffu, need)) continue;
-                const int cb = cid(g, a, b, 0);
-                uint32_t s0 = 0, s1 = 0, sz0 = 0;
-                if (need) {
-                    s0 = __ldg(cl.off + cb + klo); s1 = __ldg(cl.off + cb + khi + 1);
-                    sz0 = hz ? __ldg(cl.off + cb + min(k, khi) + 1) : s0;
-                }
-                // the warp's range: from lane 0's first particle to the largest end
-                const uint32_t A = __shfl_sync(0xffffffffu, s0, 0);
-                const uint32_t B = __reduce_max_sync(0xffffffffu, need ? s1 : A);
-                for (uint32_t c0 = A; c0 < B; c0 += CAP) {
-                    const uint32_t n = min(B - c0, (uint32_t)CAP);
-                    __syncwarp();
-                    for (uint32_t u = lane; u < n; u += 32) {
-                        const float4 q = __ldg(pos + c0 + u);
-                        const int f = pflag(q);
-                        const float3 ps = mk3(q.x, q.y, q.z) * scale;
-                        sp[p2g_slot(u)] = make_float4(ps.x, ps.y, ps.z, (f == MP_TYPEFLUID || f == MP_TYPESOLID) ? 1.0f : 0.0f);
-                        sv[p2g_slot(u)] = __ldg(vel + c0 + u);
+        const bool hx = act && (j < g.NY && k < g.NZ), hy = act && (i < g.NX && k < g.NZ), hz = act && (i < g.NX && j < g.NY);
+        FaceSums F;
+        bool near = true;
+        if (AIR) {
+            near = false;
+            if (act) {
+                const int bw = (g.NZ + 3) / 4, bh = (g.NY + 3) / 4;
+                const int bi0 = max(i - R, 0) >> 2, bi1 = min(i + R, g.NX - 1) >> 2;
+                const int bj0 = max(j - R, 0) >> 2, bj1 = min(j + R, g.NY - 1) >> 2;
+                const int bk0 = max(k - R, 0) >> 2, bk1 = min(k + R, g.NZ - 1) >> 2;
+                for (int bi = bi0; bi <= bi1; bi++)
+                    for (int bj = bj0; bj <= bj1; bj++)
+                        for (int bk = bk0; bk <= bk1; bk++) {
+                            const int br = (bi * bh + bj) * bw + bk;
+                            near |= (__ldg(air_brick + (br >> 5)) >> (br & 31)) & 1u;
+                        }
+            }
+        }
+        if (__any_sync(0xffffffffu, near)) {
+            const float3 gpx = mk3((float)i, (float)j + 0.5f, (float)k + 0.5f);
+            const float3 gpy = mk3((float)i + 0.5f, (float)j, (float)k + 0.5f);
+            const float3 gpz = mk3((float)i + 0.5f, (float)j + 0.5f, (float)k);
+            const int klo = max(k - R, 0), khi = min(k + R, g.NZ - 1);
+            for (int di = -R; di <= R; di++) {
+                int a = i + di; if (a < 0 || a > g.NX - 1) continue;
+                const bool ax = hx && di <= HI;
+                for (int dj = -R; dj <= R; dj++) {
+                    int b = j + dj; if (b < 0 || b > g.NY - 1) continue;
+                    const bool ay = hy && dj <= HI;
+                    bool need = (ax || ay || hz) && klo <= khi;
+                    const int cb = cid(g, a, b, 0);
+                    if (AIR) {
+                        // the type mask is built at sort time; AIR <-> AIRSOLO flips since then
+                        // (markSoloAirParticle) keep the union bit valid
+                        bool any = false;
+                        if (need)
+                            for (int cc = klo; cc <= khi; cc++)
+                                any |= (__ldg(cl.tmask + cb + cc) & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO))) != 0;
+                        need = any;
                     }
-                    __syncwarp();
-                    if (!need) continue;
-                    const uint32_t lo = max(s0, c0), hi = min(s1, c0 + n);
-                    for (uint32_t p = lo; p < hi; ++p) {
-                        const float4 q = sp[p2g_slot(p - c0)];
-                        if (q.w == 0.0f) continue;
-                        const float3 ps = mk3(q.x, q.y, q.z);
-                        float3 dx = ps - gpx, dy = ps - gpy, dz = ps - gpz;
-                        float r2x = dot(dx, dx), r2y = dot(dy, dy), r2z = dot(dz, dz);
-                        bool tx = ax && r2x <= cut, ty = ay && r2y <= cut, tz = p < sz0 && r2z <= cut;
-                        if (!(tx || ty || tz)) continue;
-                        const float4 v = sv[p2g_slot(p - c0)];
-                        if (tx) { float w = v.w * sharp_kernel(r2x, 1.4f); wx += w; sx += w * v.x; }
-                        if (ty) { float w = v.w * sharp_kernel(r2y, 1.4f); wy += w; sy += w * v.y; }
-                        if (tz) { float w = v.w * sharp_kernel(r2z, 1.4f); wz += w; sz += w * v.z; }
+                    if (!__any_sync(0xffffffffu, need)) continue;
+                    uint32_t s0 = 0, s1 = 0, sz0 = 0;
+                    if (need) {
+                        s0 = __ldg(cl.off + cb + klo); s1 = __ldg(cl.off + cb + khi + 1);
+                        sz0 = hz ? __ldg(cl.off + cb + min(k + HI, khi) + 1) : s0;
+                    }
+                    // the warp's range: from the first needed particle to the largest end
+                    const uint32_t A = __reduce_min_sync(0xffffffffu, need ? s0 : 0xffffffffu);
+                    const uint32_t B = __reduce_max_sync(0xffffffffu, need ? s1 : 0u);
+                    for (uint32_t c0 = A; c0 < B; c0 += CAP) {
+                        const uint32_t n = min(B - c0, (uint32_t)CAP);
+                        uint32_t kept = 0;   // AIR: staged so far
+                        __syncwarp();
+                        // UN loads of a lane in flight together
+                        constexpr int UN = 4;
+                        for (uint32_t u0 = lane; u0 < n + lane; u0 += 32 * UN) {
+                            float4 q[UN], v[UN];
+                            #pragma unroll
+                            for (int e = 0; e < UN; e++) {
+                                const uint32_t u = u0 + 32 * e;
+                                q[e] = u < n ? __ldg(pos + c0 + u) : make_float4(0, 0, 0, flagbits(-1));
+                                if (!AIR) v[e] = u < n ? __ldg(vel + c0 + u) : q[e];
+                            }
+                            #pragma unroll
+                            for (int e = 0; e < UN; e++) {
+                                const uint32_t u = u0 + 32 * e;
+                                const int f = pflag(q[e]);
+                                const float3 ps = mk3(q[e].x, q[e].y, q[e].z) * scale;
+                                if (!AIR) {
+                                    if (u < n) {
+                                        const bool take = f == MP_TYPEFLUID || f == MP_TYPESOLID;
+                                        sp[p2g_slot(u)] = take ? make_float4(ps.x, ps.y, ps.z, 0.0f)
+                                                               : make_float4(P2G_FAR, P2G_FAR, P2G_FAR, 0.0f);
+                                        sv[p2g_slot(u)] = v[e];
+                                    }
+                                } else {
+                                    const bool take = f == MP_TYPEAIR;
+                                    const unsigned mask = __ballot_sync(0xffffffffu, take);
+                                    const uint32_t to = kept + __popc(mask & ((1u << lane) - 1u));
+                                    if (u < n) before[warp][u] = (uint16_t)to;
+                                    if (take) {
+                                        sp[p2g_slot(to)] = make_float4(ps.x, ps.y, ps.z, 0.0f);
+                                        sv[p2g_slot(to)] = __ldg(vel + c0 + u);
+                                    }
+                                    kept += __popc(mask);
+                                }
+                            }
+                        }
+                        if (AIR && lane == 0) before[warp][n] = (uint16_t)kept;
+                        __syncwarp();
+                        if (!need) continue;
+                        uint32_t lo = max(s0, c0) - c0, hi = min(s1, c0 + n) - c0, zz = min(max(sz0, c0), c0 + n) - c0;
+                        if (lo >= hi || s0 >= c0 + n || s1 <= c0) continue;
+                        if (AIR) { lo = before[warp][lo]; hi = before[warp][hi]; zz = before[warp][zz]; }
+                        p2g_walk(sp, sv, lo, hi, zz, gpx, gpy, gpz, ax ? cut : -1.0f, ay ? cut : -1.0f, hz ? cut : -1.0f, F);
                     }
                 }
             }
         }
-        if (hx) ux[fxi(g, i, j, k)] = (wx > 0) ? (sx / wx) : 0.0f;
-        if (hy) uy[fyi(g, i, j, k)] = (wy > 0) ? (sy / wy) : 0.0f;
-        if (hz) uz[fzi(g, i, j, k)] = (wz > 0) ? (sz / wz) : 0.0f;
+        if (hx) ux[fxi(g, i, j, k)] = (F.wx > 0) ? (F.sx / F.wx) : 0.0f;
+        if (hy) uy[fyi(g, i, j, k)] = (F.wy > 0) ? (F.sy / F.wy) : 0.0f;
+        if (hz) uz[fzi(g, i, j, k)] = (F.wz > 0) ? (F.sz / F.wz) : 0.0f;
     }
 }
 
@@ -319,30 +321,63 @@ __global__ void __launch_bounds__(256) k_g2p(Grid g, int np, const float4* __res
     }
 }
 
-// mapHeatp2g_hash: cell-centred, 27 cells, all particles, unweighted by mass
-__global__ void __launch_bounds__(256) k_heat_p2g(Grid g, Cells cl, const float4* __restrict__ pos,
-                                                  const float4* __restrict__ heat, float* __restrict__ Tp, float dflt) {
+// mapHeatp2g_hash: cell-centred, 27 cells, all particles, unweighted by mass.
+// Staged by warps as the water P2G: for one (di, dj) the lanes' windows along k
+// are overlapping parts of one range of the sorted particles, which the warp
+// copies with coalesced loads (scaled position and temperature); a lane's own
+// loads from global memory hit a line each. 96^3: 468 -> 200 us.
+constexpr int HEAT_CAP = 320;
+__global__ void __launch_bounds__(256, 3) k_heat_p2g(Grid g, Cells cl, const float4* __restrict__ pos,
+                                                     const float4* __restrict__ heat, float* __restrict__ Tp, float dflt) {
+    __shared__ float4 staged[8][p2g_slots(HEAT_CAP)];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4* sp = staged[warp];
+    const Tiles T = make_tiles(g.NX, g.NY, g.NZ);
     const float scale = 1.0f / g.h;
-    MP_GRID_LOOP(idx, g.n) {
-        int i, j, k; getijk(g, (int)idx, i, j, k);
-        float3 gp = mk3((float)i + 0.5f, (float)j + 0.5f, (float)k + 0.5f);
+    // every lane of a warp runs the same iterations and takes part in the staging
+    MP_GRID_LOOP(t, T.threads()) {
+        int i, j, k;
+        const bool act = tile_ijk(T, t, i, j, k);
+        if (!__any_sync(0xffffffffu, act)) continue;
+        const float3 gp = mk3((float)i + 0.5f, (float)j + 0.5f, (float)k + 0.5f);
+        const int klo = max(k - 1, 0), khi = min(k + 1, g.NZ - 1);
         float ws = 0, hs = 0;
-        for (int di = -1; di <= 1; di++) {
-            int a = i + di; if (a < 0 || a > g.NX - 1) continue;
-            for (int dj = -1; dj <= 1; dj++) {
-                int b = j + dj; if (b < 0 || b > g.NY - 1) continue;
-                int k0 = max(k - 1, 0), k1 = min(k + 1, g.NZ - 1);
-                uint32_t s0 = __ldg(cl.off + cid(g, a, b, k0)), s1 = __ldg(cl.off + cid(g, a, b, k1) + 1);
-                for (uint32_t p = s0; p < s1; ++p) {
-                    float4 q = __ldg(pos + p);
-                    float3 d = mk3(q.x, q.y, q.z) * scale - gp;
-                    float w = sharp_kernel(dot(d, d), 1.4f);
-                    ws += w;
-                    hs += w * __ldg(&heat[p].x);
+        for (int a = max(i - 1, 0); a <= min(i + 1, g.NX - 1); a++)
+            for (int b = max(j - 1, 0); b <= min(j + 1, g.NY - 1); b++) {
+                const int cb = cid(g, a, b, 0);
+                uint32_t s0 = 0, s1 = 0;
+                if (act) { s0 = __ldg(cl.off + cb + klo); s1 = __ldg(cl.off + cb + khi + 1); }
+                const uint32_t A = __shfl_sync(0xffffffffu, s0, 0);   // lane 0 holds the lowest k
+                const uint32_t B = __reduce_max_sync(0xffffffffu, act ? s1 : A);
+                for (uint32_t c0 = A; c0 < B; c0 += HEAT_CAP) {
+                    const uint32_t n = min(B - c0, (uint32_t)HEAT_CAP);
+                    __syncwarp();
+                    constexpr int UN = 4;   // loads of a lane in flight together
+                    for (uint32_t u0 = lane; u0 < n; u0 += 32 * UN) {
+                        float4 q[UN];
+                        #pragma unroll
+                        for (int e = 0; e < UN; e++)
+                            if (u0 + 32 * e < n) { q[e] = __ldg(pos + c0 + u0 + 32 * e); q[e].w = __ldg(&heat[c0 + u0 + 32 * e].x); }
+                        #pragma unroll
+                        for (int e = 0; e < UN; e++)
+                            if (u0 + 32 * e < n) {
+                                const float3 ps = mk3(q[e].x, q[e].y, q[e].z) * scale;
+                                sp[p2g_slot(u0 + 32 * e)] = make_float4(ps.x, ps.y, ps.z, q[e].w);
+                            }
+                    }
+                    __syncwarp();
+                    if (!act) continue;
+                    const uint32_t lo = max(s0, c0), hi = min(s1, c0 + n);
+                    for (uint32_t p = lo; p < hi; ++p) {
+                        const float4 q = sp[p2g_slot(p - c0)];
+                        const float3 d = mk3(q.x, q.y, q.z) - gp;
+                        const float w = sharp_kernel14(dot(d, d));
+                        ws += w;
+                        hs += w * q.w;
+                    }
                 }
             }
-        }
-        Tp[idx] = (ws > 0) ? (hs / ws) : dflt;
+        if (act) Tp[cid(g, i, j, k)] = (ws > 0) ? (hs / ws) : dflt;
     }
 }
 
@@ -387,14 +422,15 @@ static Cells cells_of(MpCtx* c) { return Cells{c->cell_off, c->tmask}; }
 int k_p2g_faces(MpCtx* c, float** out, int which) {
     const Grid& g = c->G;
     long long tot = make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1).threads();
-    if (which == 0) {
-        const int smem = 8 * 2 * p2g_slots(P2G_CAP) * (int)sizeof(float4);
-        MP_CUDA(c, cudaFuncSetAttribute(k_p2g_water<P2G_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        k_p2g_water<P2G_CAP><<<mp_blocks(tot, 256), 256, smem, c->stream>>>(g, cells_of(c), c->pos, c->vel, out[0], out[1], out[2]);
-    }
-    else
-        k_p2g_air<<<mp_blocks(tot, 256), 256, 0, c->stream>>>(g, cells_of(c), c->pos, c->vel, out[0], out[1], out[2],
-                                                              c->air_brick);
+    auto run = [&](auto kern, int cap) -> int {
+        const int smem = 8 * 2 * p2g_slots(cap) * (int)sizeof(float4);
+        MP_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kern<<<mp_blocks(tot, 256), 256, smem, c->stream>>>(g, cells_of(c), c->pos, c->vel, out[0], out[1], out[2],
+                                                            c->air_brick);
+        return MP_OK;
+    };
+    if (which == 0) MP_TRY(run(k_p2g_staged<false, P2G_CAP>, P2G_CAP));
+    else MP_TRY(run(k_p2g_staged<true, P2G_AIR_CAP>, P2G_AIR_CAP));
     c->launches++;
     MP_CHECK_LAUNCH(c);
     return MP_OK;
@@ -494,8 +530,9 @@ int k_g2p(MpCtx* c) {
 }
 
 int k_heat_p2g_launch(MpCtx* c) {
-    k_heat_p2g<<<mp_blocks(c->G.n, 256), 256, 0, c->stream>>>(c->G, cells_of(c), c->pos, c->heat, c->Tp,
-                                                              c->P.default_temperature);
+    const long long tot = make_tiles(c->G.NX, c->G.NY, c->G.NZ).threads();
+    k_heat_p2g<<<mp_blocks(tot, 256), 256, 0, c->stream>>>(c->G, cells_of(c), c->pos, c->heat, c->Tp,
+                                                           c->P.default_temperature);
     c->launches++;
     MP_CHECK_LAUNCH(c);
     return MP_OK;
