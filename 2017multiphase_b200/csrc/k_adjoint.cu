@@ -38,6 +38,7 @@
 // the first replay are kept per step, so the recomputations neither splat
 // nor solve).
 #include "ctx.cuh"
+#include "p2g_walk.cuh"
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -385,6 +386,119 @@ __global__ void __launch_bounds__(256) k_ad_p2g_w(Grid g, const uint32_t* __rest
         if (hy) { const int f = fyi(g, i, j, k); W.y[f] = wy; u.y[f] = wy > (T)0 ? sy / wy : (T)0; }
         if (hz) { const int f = fzi(g, i, j, k); W.z[f] = wz; u.z[f] = wz > (T)0 ? sz / wz : (T)0; }
     }
+}
+// The same splat in FP32 with the engine's pair loop (p2g_walk): a column's
+// records fit one chunk, a lane's staging loads go out four at a time, and in
+// the air splat (PH 1) only the phase's records are staged. Per launch at 64^3
+// (dam) 225 -> DAM_P2G us, at 96^3 (column) water 1290 -> COL_P2GW us, air 770
+// -> COL_P2GA us against k_ad_p2g_w, which stays for FP64.
+template <int PH, int CAP>
+__global__ void __launch_bounds__(256, PH ? 3 : 2) k_ad_p2g_f(Grid g, const uint32_t* __restrict__ off,
+                                                              const float4* __restrict__ xs4, const float4* __restrict__ vs4,
+                                                              Fc<float> u, Fc<float> W, const uint8_t* __restrict__ cellmask) {
+    using Wn = SplatWin<PH>;
+    constexpr int R = Wn::AC;
+    extern __shared__ float4 adp_sm[];
+    __shared__ uint16_t before[PH ? 8 : 1][PH ? CAP + 2 : 1];   // the phase's records of the chunk before each place
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4* sp = adp_sm + (size_t)warp * 2 * p2g_slots(CAP);
+    float4* sv = sp + p2g_slots(CAP);
+    const Tiles Tl = make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1);
+    const float scale = 1.0f / g.h;
+    const float cut = (1.4f * 1.4f) * 1.0001f;
+    MP_GRID_LOOP(t, Tl.threads()) {
+        int i, j, k;
+        const bool act = tile_ijk(Tl, t, i, j, k);
+        if (!__any_sync(0xffffffffu, act)) continue;
+        const bool hx = act && j < g.NY && k < g.NZ, hy = act && i < g.NX && k < g.NZ, hz = act && i < g.NX && j < g.NY;
+        FaceSums F;
+        const float3 gpx = mk3((float)i, (float)j + 0.5f, (float)k + 0.5f);
+        const float3 gpy = mk3((float)i + 0.5f, (float)j, (float)k + 0.5f);
+        const float3 gpz = mk3((float)i + 0.5f, (float)j + 0.5f, (float)k);
+        const int klo = max(k - R, 0), khi = min(k + R, g.NZ - 1), kzhi = min(k + Wn::HI, g.NZ - 1);
+        for (int di = -R; di <= R; di++) {
+            const int a = i + di;
+            if (a < 0 || a > g.NX - 1) continue;   // the same for the whole warp
+            const bool ax = hx && di >= -Wn::LO && di <= Wn::HI;
+            for (int dj = -R; dj <= R; dj++) {
+                const int b = j + dj;
+                if (b < 0 || b > g.NY - 1) continue;
+                const bool ay = hy && dj >= -Wn::LO && dj <= Wn::HI;
+                bool need = (ax || ay || hz) && klo <= khi;
+                const int cb = cid(g, a, b, 0);
+                if (need && cellmask) {
+                    bool any = false;
+                    for (int cc = klo; cc <= khi; cc++) any = any || cellmask[cb + cc];
+                    need = any;
+                }
+                if (!__any_sync(0xffffffffu, need)) continue;
+                uint32_t s0 = 0, s1 = 0, sz1 = 0;
+                if (need) {
+                    s0 = off[cb + klo]; s1 = off[cb + khi + 1];
+                    sz1 = hz ? off[cb + kzhi + 1] : s0;
+                }
+                const uint32_t A = __reduce_min_sync(0xffffffffu, need ? s0 : 0xffffffffu);
+                const uint32_t B = __reduce_max_sync(0xffffffffu, need ? s1 : 0u);
+                for (uint32_t c0 = A; c0 < B; c0 += CAP) {
+                    const uint32_t n = min(B - c0, (uint32_t)CAP);
+                    uint32_t kept = 0;
+                    __syncwarp();
+                    constexpr int UN = 4;   // loads of a lane in flight together
+                    for (uint32_t u0 = lane; u0 < n + lane; u0 += 32 * UN) {
+                        float4 q[UN], v[UN];
+                        #pragma unroll
+                        for (int e = 0; e < UN; e++) {
+                            const uint32_t uu = u0 + 32 * e;
+                            q[e] = uu < n ? __ldg(xs4 + c0 + uu) : make_float4(0, 0, 0, 0);
+                            v[e] = uu < n ? __ldg(vs4 + c0 + uu) : q[e];
+                        }
+                        #pragma unroll
+                        for (int e = 0; e < UN; e++) {
+                            const uint32_t uu = u0 + 32 * e;
+                            const bool on = q[e].w != 0.0f;   // mass 0: the other phase, adds nothing
+                            const float3 ps = mk3(q[e].x, q[e].y, q[e].z) * scale;
+                            v[e].w = q[e].w;
+                            uint32_t to = uu;
+                            if (PH) {
+                                const unsigned mask = __ballot_sync(0xffffffffu, on);
+                                to = kept + __popc(mask & ((1u << lane) - 1u));
+                                if (uu < n) before[warp][uu] = (uint16_t)to;
+                                kept += __popc(mask);
+                            }
+                            if (PH ? on : uu < n) {
+                                sp[p2g_slot(to)] = on ? make_float4(ps.x, ps.y, ps.z, 0.0f) : make_float4(P2G_FAR, P2G_FAR, P2G_FAR, 0.0f);
+                                sv[p2g_slot(to)] = v[e];
+                            }
+                        }
+                    }
+                    if (PH && lane == 0) before[warp][n] = (uint16_t)kept;
+                    __syncwarp();
+                    if (!need || s0 >= c0 + n || s1 <= c0) continue;
+                    uint32_t lo = max(s0, c0) - c0, hi = min(s1, c0 + n) - c0, zz = min(max(sz1, c0), c0 + n) - c0;
+                    if (PH) { lo = before[warp][lo]; hi = before[warp][hi]; zz = before[warp][zz]; }
+                    p2g_walk(sp, sv, lo, hi, zz, gpx, gpy, gpz, ax ? cut : -1.0f, ay ? cut : -1.0f, hz ? cut : -1.0f, F);
+                }
+            }
+        }
+        if (hx) { const int f = fxi(g, i, j, k); W.x[f] = F.wx; u.x[f] = F.wx > 0 ? F.sx / F.wx : 0.0f; }
+        if (hy) { const int f = fyi(g, i, j, k); W.y[f] = F.wy; u.y[f] = F.wy > 0 ? F.sy / F.wy : 0.0f; }
+        if (hz) { const int f = fzi(g, i, j, k); W.z[f] = F.wz; u.z[f] = F.wz > 0 ? F.sz / F.wz : 0.0f; }
+    }
+}
+template <class T, int PH>
+int ad_p2g(MpCtx* c, const Grid& g, const uint32_t* off, const T* xs4, const T* vs4, Fc<T> u, Fc<T> W,
+           const uint8_t* cellmask) {
+    const int nb = mp_blocks(make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1).threads(), 256);
+    if constexpr (sizeof(T) == 4) {
+        constexpr int CAP = PH ? 192 : 320;
+        const int smem = 8 * 2 * p2g_slots(CAP) * (int)sizeof(float4);
+        MP_CUDA(c, cudaFuncSetAttribute(k_ad_p2g_f<PH, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k_ad_p2g_f<PH, CAP><<<nb, 256, smem, c->stream>>>(g, off, reinterpret_cast<const float4*>(xs4),
+                                                          reinterpret_cast<const float4*>(vs4), u, W, cellmask);
+    } else {
+        k_ad_p2g_w<T, PH><<<nb, 256, 0, c->stream>>>(g, off, xs4, vs4, u, W, cellmask);
+    }
+    return MP_OK;
 }
 // particle records in a step's recorded sorted order: (a xyz, mass or 0) and
 // (b xyz, 0), so the face gathers read contiguous records within a cell
@@ -977,19 +1091,41 @@ __global__ void k_ad_g2p_adj_p(Grid g, int np, const uint32_t* __restrict__ orde
 // 3x3x3 cells around its node, i.e. near a particle whose replay cell is not
 // its recorded one. Membership is decided from the replay's own positions, and
 // a face adds its members in (a, b, c, particle) order in either window.
-// A warp handles 32 nodes along k (i, j fixed), a thread a node's three
-// faces, with the candidates of each column (a, b) staged in shared memory
-// as in k_ad_p2g_w.
+// A warp handles 32 nodes along k (i, j fixed), a thread a node's three faces.
+// For each column (a, b) the warp stages the candidates once with what all its
+// lanes share: whether a candidate's stencil holds faces of this (i, j) at all
+// (those that do not are dropped, their places closed up by a running count, so
+// that a lane's part stays a range), the product of its two weights across k for
+// each face, and its base and weights along k. A lane then only tests its k and
+// multiplies. Forming all of it in every lane took 105 instructions a candidate
+// (three divisions by h, three bases), this about 27: per launch at 64^3 (dam)
+// 1200 -> DAM_G2P us, at 96^3 (column) 1460 -> COL_G2P us.
+template <class T> struct G2pRec {   // one candidate; u/v: base along k and flags as bits
+    alignas(16) T a[4];              // weight products of the x-, y- and z-face; base of the half coordinate | flags 28, 29
+    alignas(16) T v[4];              // cotangent; base of the full coordinate | flag 28
+    alignas(16) T f[4];              // weights along k of faces base, base + 1: half, full coordinate
+};
+__device__ __forceinline__ float g2p_bits(float, int v) { return __int_as_float(v); }
+__device__ __forceinline__ double g2p_bits(double, int v) { return __hiloint2double(0, v); }
+__device__ __forceinline__ int g2p_int(float v) { return __float_as_int(v); }
+__device__ __forceinline__ int g2p_int(double v) { return __double2loint(v); }
+template <class T> __host__ __device__ constexpr int g2p_cap() { return sizeof(T) == 4 ? 224 : 96; }
 template <class T>
-__global__ void __launch_bounds__(256) k_ad_g2p_adj_w(Grid g, const uint32_t* __restrict__ off,
-                                                      const T* __restrict__ xs4, const T* __restrict__ vgs4, Fc<T> q,
-                                                      const uint8_t* __restrict__ cellmask,
-                                                      const uint8_t* __restrict__ near) {
-    constexpr int CAP = sizeof(T) == 4 ? 128 : 64;
-    __shared__ T sm_x[8][CAP][4];
-    __shared__ T sm_v[8][CAP][4];
+__global__ void __launch_bounds__(256, 2) k_ad_g2p_adj_w(Grid g, const uint32_t* __restrict__ off,
+                                                         const T* __restrict__ xs4, const T* __restrict__ vgs4, Fc<T> q,
+                                                         const uint8_t* __restrict__ cellmask,
+                                                         const uint8_t* __restrict__ near) {
+    constexpr int CAP = g2p_cap<T>();
+    extern __shared__ __align__(16) unsigned char g2p_raw[];
+    __shared__ uint16_t before[8][CAP + 2];   // candidates kept before each place of the chunk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    G2pRec<T>* rec = reinterpret_cast<G2pRec<T>*>(g2p_raw) + (size_t)warp * CAP;
     const Tiles Tl = make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1);
+    // one axis of a stencil: clamped position on an array of n faces or cells,
+    // its base; the weight of face e if the stencil holds it
+    auto clampx = [](T p, int n) { return p < (T)0 ? (T)0 : (p > (T)n ? (T)n : p); };
+    auto base = [](T p, int n) { return (int)(p < (T)(n - 2) ? p : (T)(n - 2)); };
+    auto wt = [](T p, int b, int e) { return e ? p - (T)b : (T)(b + 1) - p; };
     MP_GRID_LOOP(t, Tl.threads()) {
         int i, j, k;
         const bool act = tile_ijk(Tl, t, i, j, k);
@@ -1005,7 +1141,6 @@ __global__ void __launch_bounds__(256) k_ad_g2p_adj_w(Grid g, const uint32_t* __
         const int R = __reduce_max_sync(0xffffffffu, act ? AC : 1);
         T qx = 0, qy = 0, qz = 0;
         const int klo = max(k - AC, 0), khi = min(k + AC, g.NZ - 1), kzhi = min(k + HI, g.NZ - 1);
-        const int W0 = g.NX + 1, H1 = g.NY + 1, D2 = g.NZ + 1;
         for (int di = -R; di <= R; di++) {
             const int a = i + di;
             if (a < 0 || a > g.NX - 1) continue;   // the same for the whole warp
@@ -1033,38 +1168,62 @@ __global__ void __launch_bounds__(256) k_ad_g2p_adj_w(Grid g, const uint32_t* __
                 const uint32_t B = __reduce_max_sync(0xffffffffu, need ? s1 : 0u);
                 for (uint32_t c0 = A; c0 < B; c0 += CAP) {
                     const uint32_t n = min(B - c0, (uint32_t)CAP);
+                    uint32_t kept = 0;
                     __syncwarp();
-                    for (uint32_t e = lane; e < n; e += 32) {
-                        const T* r = xs4 + 4 * (size_t)(c0 + e);
-                        const T* v = vgs4 + 4 * (size_t)(c0 + e);
-                        sm_x[warp][e][0] = r[0]; sm_x[warp][e][1] = r[1]; sm_x[warp][e][2] = r[2];
-                        sm_v[warp][e][0] = v[0]; sm_v[warp][e][1] = v[1]; sm_v[warp][e][2] = v[2];
-                    }
-                    __syncwarp();
-                    if (!need) continue;
-                    const uint32_t lo = max(s0, c0), hi = min(s1, c0 + n);
-                    for (uint32_t p = lo; p < hi; ++p) {
-                        const T X = sm_x[warp][p - c0][0] / (T)g.h, Y = sm_x[warp][p - c0][1] / (T)g.h;
-                        const T Z = sm_x[warp][p - c0][2] / (T)g.h;
+                    constexpr int UN = 2;   // loads of a lane in flight together
+                    for (uint32_t u0 = lane; u0 < n + lane; u0 += 32 * UN) {
+                        T px[UN][3], pv[UN][3];
                         #pragma unroll
-                        for (int f = 0; f < 3; f++) {
-                            const bool on = f == 0 ? axc : (f == 1 ? ay : (azc && p < sz1));
-                            if (!on) continue;
-                            const int w = f == 0 ? W0 : g.NX, hh = f == 1 ? H1 : g.NY, d = f == 2 ? D2 : g.NZ;
-                            T px, py, pz; ipos(f, X, Y, Z, px, py, pz);
-                            px = px < (T)0 ? (T)0 : (px > (T)w ? (T)w : px);
-                            py = py < (T)0 ? (T)0 : (py > (T)hh ? (T)hh : py);
-                            pz = pz < (T)0 ? (T)0 : (pz > (T)d ? (T)d : pz);
-                            const int bi = (int)(px < (T)(w - 2) ? px : (T)(w - 2));
-                            const int bj = (int)(py < (T)(hh - 2) ? py : (T)(hh - 2));
-                            const int bk = (int)(pz < (T)(d - 2) ? pz : (T)(d - 2));
-                            const int ei = i - bi, ej = j - bj, ek = k - bk;
-                            if (ei < 0 || ei > 1 || ej < 0 || ej > 1 || ek < 0 || ek > 1) continue;
-                            const T fx = ei ? px - (T)bi : (T)(bi + 1) - px, fy = ej ? py - (T)bj : (T)(bj + 1) - py;
-                            const T fz = ek ? pz - (T)bk : (T)(bk + 1) - pz;
-                            const T term = fx * fy * fz * sm_v[warp][p - c0][f];
-                            if (f == 0) qx += term; else if (f == 1) qy += term; else qz += term;
+                        for (int e = 0; e < UN; e++) {
+                            const uint32_t u = u0 + 32 * e;
+                            const size_t s = 4 * (size_t)(c0 + (u < n ? u : 0));
+                            #pragma unroll
+                            for (int d = 0; d < 3; d++) { px[e][d] = xs4[s + d]; pv[e][d] = vgs4[s + d]; }
                         }
+                        #pragma unroll
+                        for (int e = 0; e < UN; e++) {
+                            const uint32_t u = u0 + 32 * e;
+                            const T X = px[e][0] / (T)g.h, Y = px[e][1] / (T)g.h, Z = px[e][2] / (T)g.h;
+                            const T half = (T)0.5f;
+                            const T xf = clampx(X, g.NX + 1), xh = clampx(X - half, g.NX);
+                            const T yf = clampx(Y, g.NY + 1), yh = clampx(Y - half, g.NY);
+                            const T zf = clampx(Z, g.NZ + 1), zh = clampx(Z - half, g.NZ);
+                            const int bxf = base(xf, g.NX + 1), bxh = base(xh, g.NX), byf = base(yf, g.NY + 1), byh = base(yh, g.NY);
+                            const int bzf = base(zf, g.NZ + 1), bzh = base(zh, g.NZ);
+                            auto in = [](int d) { return d == 0 || d == 1; };
+                            const bool m0 = in(i - bxf) && in(j - byh), m1 = in(i - bxh) && in(j - byf), m2 = in(i - bxh) && in(j - byh);
+                            const bool keep = u < n && (m0 || m1 || m2);
+                            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+                            const uint32_t to = kept + __popc(mask & ((1u << lane) - 1u));
+                            if (u < n) before[warp][u] = (uint16_t)to;
+                            if (keep) {
+                                G2pRec<T>& r = rec[to];
+                                const T wxh = wt(xh, bxh, i - bxh), wyh = wt(yh, byh, j - byh);
+                                r.a[0] = wt(xf, bxf, i - bxf) * wyh; r.a[1] = wxh * wt(yf, byf, j - byf); r.a[2] = wxh * wyh;
+                                r.a[3] = g2p_bits((T)0, bzh | (m0 ? 1 << 28 : 0) | (m1 ? 1 << 29 : 0));
+                                r.v[0] = pv[e][0]; r.v[1] = pv[e][1]; r.v[2] = pv[e][2];
+                                r.v[3] = g2p_bits((T)0, bzf | (m2 ? 1 << 28 : 0));
+                                r.f[0] = wt(zh, bzh, 0); r.f[1] = wt(zh, bzh, 1); r.f[2] = wt(zf, bzf, 0); r.f[3] = wt(zf, bzf, 1);
+                            }
+                            kept += __popc(mask);
+                        }
+                    }
+                    if (lane == 0) before[warp][n] = (uint16_t)kept;
+                    __syncwarp();
+                    if (!need || s0 >= c0 + n || s1 <= c0) continue;
+                    const uint32_t lo = before[warp][max(s0, c0) - c0], hi = before[warp][min(s1, c0 + n) - c0],
+                                   zz = before[warp][min(max(sz1, c0), c0 + n) - c0];
+                    #pragma unroll 2
+                    for (uint32_t p = lo; p < hi; ++p) {
+                        const G2pRec<T>& r = rec[p];
+                        const int bh = g2p_int(r.a[3]), bf = g2p_int(r.v[3]);
+                        const int eh = k - (bh & 0xfffffff), ef = k - (bf & 0xfffffff);
+                        const T fh = eh ? r.f[1] : r.f[0], ff = ef ? r.f[3] : r.f[2];
+                        const bool ih = (unsigned)eh <= 1u, iz = (unsigned)ef <= 1u;
+                        const T tx = r.a[0] * fh * r.v[0], ty = r.a[1] * fh * r.v[1], tz = r.a[2] * ff * r.v[2];
+                        if (axc && ih && (bh & (1 << 28))) qx += tx;
+                        if (ay && ih && (bh & (1 << 29))) qy += ty;
+                        if (azc && p < zz && iz && (bf & (1 << 28))) qz += tz;
                     }
                 }
             }
@@ -1074,6 +1233,19 @@ __global__ void __launch_bounds__(256) k_ad_g2p_adj_w(Grid g, const uint32_t* __
         if (hz) q.z[fzi(g, i, j, k)] = qz;
     }
 }
+template <class T>
+int ad_g2p_adj(MpCtx* c, const Grid& g, const uint32_t* off, const T* xs4, const T* vgs4, Fc<T> q,
+               const uint8_t* cellmask, const uint8_t* near) {
+    const int nb = mp_blocks(make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1).threads(), 256);
+    const int smem = 8 * g2p_cap<T>() * (int)sizeof(G2pRec<T>);
+    MP_CUDA(c, cudaFuncSetAttribute(k_ad_g2p_adj_w<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_ad_g2p_adj_w<T><<<nb, 256, smem, c->stream>>>(g, off, xs4, vgs4, q, cellmask, near);
+    return MP_OK;
+}
+// the splat kernel's two quotients, 1.96 / r2 and that over r2 again, for r2 in
+// [1e-4, 1.96]: both equal / on every float of that range
+__device__ __forceinline__ float ad_quot(float a, float r2) { return quot_in_range(a, r2); }
+__device__ __forceinline__ double ad_quot(double a, double r2) { return a / r2; }
 // per face ub/W of a splat (0 where the face took no weight): the factor every
 // particle of the face's window takes
 template <class T>
@@ -1111,30 +1283,45 @@ __global__ void k_ad_p2g_adj(Grid g, int np, const uint32_t* __restrict__ order,
                 if (fi < 0 || fi >= W_) continue;
                 for (int fj = j0; fj <= j1; fj++) {
                     if (fj < 0 || fj >= H_) continue;
-                    for (int fk = k0; fk <= k1; fk++) {
-                        if (fk < 0 || fk >= D_) continue;
+                    // a row of faces along k: the distances and the loads of all
+                    // of them first (the loads of one face after another, each
+                    // behind its branch, were most of the time), then the terms
+                    // in order
+                    constexpr int NK = 2 * Wn::AC + 1;
+                    T dxs[1], r2s[NK], as[NK], us[NK], dzs[NK];
+                    T dy = 0;
+                    #pragma unroll
+                    for (int e = 0; e < NK; e++) {
+                        const int fk = k0 + e;
                         float gx, gy, gz; face_pos(ax, fi, fj, fk, gx, gy, gz);
-                        T dx = X - (T)gx, dy = Y - (T)gy, dz = Z - (T)gz;
-                        T r2 = dx * dx + dy * dy + dz * dz;
+                        dxs[0] = X - (T)gx; dy = Y - (T)gy; dzs[e] = Z - (T)gz;
+                        r2s[e] = dxs[0] * dxs[0] + dy * dy + dzs[e] * dzs[e];
                         // beyond the kernel radius the weight and its slope are zero
-                        if (!(r2 < cker)) continue;
-                        const int f = face_index(g, ax, fi, fj, fk);
-                        // ub/W of the face (0 where the face took no weight)
-                        const T a = fsel(ubw, ax)[f];
+                        const bool on = fk <= k1 && fk >= 0 && fk < D_ && r2s[e] < cker;
+                        as[e] = 0; us[e] = 0;
+                        if (on) {
+                            const int f = face_index(g, ax, fi, fj, fk);
+                            as[e] = __ldg(fsel(ubw, ax) + f);   // ub/W of the face (0 where the face took no weight)
+                            us[e] = __ldg(fsel(u, ax) + f);
+                        }
+                    }
+                    #pragma unroll
+                    for (int e = 0; e < NK; e++) {
+                        const T a = as[e], r2 = r2s[e];
                         if (a == (T)0) continue;
                         // the kernel c/r2 - 1 and its slope -c/r2^2 (zero below
                         // the clamp at r2 = 1e-4) from one division
                         T k_, kd;
                         if (r2 > (T)0.0001f) {
-                            const T qv = cker / r2;
-                            k_ = qv - (T)1; kd = -qv / r2;
+                            const T qv = ad_quot(cker, r2);
+                            k_ = qv - (T)1; kd = -ad_quot(qv, r2);
                             if (!(k_ > (T)0)) continue;
                         } else {
                             k_ = cker / (T)0.0001f - (T)1; kd = (T)0;
                         }
                         vb[ax] += a * m * k_;
-                        const T sv = (pv - fsel(u, ax)[f]) * a * m * kd * (T)2 * scale;
-                        gxs += sv * dx; gys += sv * dy; gzs += sv * dz;
+                        const T sv = (pv - us[e]) * a * m * kd * (T)2 * scale;
+                        gxs += sv * dxs[0]; gys += sv * dy; gzs += sv * dzs[e];
                     }
                 }
             }
@@ -1856,14 +2043,14 @@ template <class T> static int fwd_step(const Replay<T>& R, int k, const T* x, co
     if (splat) {
         k_ad_slot_gather<T><<<nbp, 256, 0, s>>>(R.np, t->order[k], x, I.va, air ? t->mass_w : t->mass, R.a(W_S4A),
                                                 R.a(W_S4B));
-        k_ad_p2g_w<T, 0><<<nbw, 256, 0, s>>>(g, t->off[k], R.a(W_S4A), R.a(W_S4B), I.up, I.wt, nullptr);
+        MP_TRY((ad_p2g<T, 0>(c, g, t->off[k], R.a(W_S4A), R.a(W_S4B), I.up, I.wt, nullptr)));
     }
     if (air) {
         uint8_t* airc = static_cast<uint8_t*>(t->wk[W_AIRC]);
         k_ad_air_cells<<<nbc, 256, 0, s>>>(g.n, t->off[k], t->order[k], t->phase, airc);
         if (splat) {
             k_ad_slot_gather<T><<<nbp, 256, 0, s>>>(R.np, t->order[k], x, I.va, t->mass_a, R.a(W_S4C), R.a(W_S4B));
-            k_ad_p2g_w<T, 1><<<nbw, 256, 0, s>>>(g, t->off[k], R.a(W_S4C), R.a(W_S4B), I.upa, I.wta, airc);
+            MP_TRY((ad_p2g<T, 1>(c, g, t->off[k], R.a(W_S4C), R.a(W_S4B), I.upa, I.wta, airc)));
         }
         k_ad_sweepu_s<T><<<nbf, 256, 0, s>>>(g, I.upa, R.f(W_T0), I.sela, I.swa);
         k_ad_sweepu_s<T><<<nbf, 256, 0, s>>>(g, R.f(W_T0), R.f(W_A0), I.sela, I.swa);
@@ -1966,11 +2153,11 @@ template <class T> static int adj_step(const Replay<T>& R, int k, const T* x, co
     }
     // q = I^T vgbar on B0 (A0 for the air faces); ufbar = q, uoldbar = -cdu q
     const int nbw = mp_blocks(make_tiles(g.NX + 1, g.NY + 1, g.NZ + 1).threads(), 256);
-    k_ad_g2p_adj_w<T><<<nbw, 256, 0, s>>>(g, t->off[k], R.a(W_S4A), R.a(W_S4B), R.f(W_B0), nullptr, nearp);
+    MP_TRY(ad_g2p_adj<T>(c, g, t->off[k], R.a(W_S4A), R.a(W_S4B), R.f(W_B0), nullptr, nearp));
     if (air) {
         // the air cell mask of this step, from its forward replay
         const uint8_t* airc = static_cast<const uint8_t*>(t->wk[W_AIRC]);
-        k_ad_g2p_adj_w<T><<<nbw, 256, 0, s>>>(g, t->off[k], R.a(W_S4A), R.a(W_S4C), R.f(W_A0), airc, nearp);
+        MP_TRY(ad_g2p_adj<T>(c, g, t->off[k], R.a(W_S4A), R.a(W_S4C), R.f(W_A0), airc, nearp));
     }
     const T cdu = alpha == (T)1 ? (T)1 : alpha;
     // wall rules then the two passes, transposed (B0 -> B1 -> T0 -> B1); the
