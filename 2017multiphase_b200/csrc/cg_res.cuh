@@ -420,8 +420,8 @@ inline size_t res_smem(const ResGeom& t) {
     return 16 * (size_t)t.KG * ((size_t)(t.ti + 2) * (t.tj + 2) + (size_t)t.ti * t.tj + hrows) + 8 * hrows;
 }
 // The tiling with the least work for the busiest thread: about 100 issue slots
-// for an own group (three passes over it), 50 for a halo group, and 10 for
-// each CTA that all the others poll. nblk = 0 when no tiling fits the SMs'
+// for an own group (three passes over it), 50 for a halo group, and 2 for
+// each CTA that all the others poll (its slot's line apart, that is nearly free). nblk = 0 when no tiling fits the SMs'
 // registers and shared memory.
 template <class R> inline ResPlan res_plan(const Grid& g, int sms, size_t smem_max) {
     ResPlan best;
@@ -439,7 +439,7 @@ template <class R> inline ResPlan res_plan(const Grid& g, int sms, size_t smem_m
             const ResGeom t{ti, tj, nbi, nbj, KG};
             const size_t sm = res_smem(t);
             if (sm > smem_max) continue;
-            const double cost = (100.0 * ng + 50.0 * nhg) / 128.0 + 10.0 * nbi * nbj;
+            const double cost = (100.0 * ng + 50.0 * nhg) / 128.0 + 2.0 * nbi * nbj;
             if (cost < best_cost) {
                 best_cost = cost;
                 best.g = t; best.nblk = nbi * nbj; best.Q = Q; best.smem = sm;

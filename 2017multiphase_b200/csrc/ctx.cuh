@@ -90,6 +90,10 @@ struct MpCtx {
     uint8_t *tmask = 0;
     uint32_t *air_brick = 0;     // bit per brick (4^3 cells, 8^3 of the 2x grid) holding an AIR/AIRSOLO particle (last sort)
     size_t air_brick_words = 0;
+    // a bit per cell of the simulation grid (last sort), a spare word before and
+    // after: AIR/AIRSOLO, then FLUID/SOLID cell_bits_half words further
+    uint32_t *cell_bits = 0;
+    size_t cell_bits_half = 0;
     uint32_t *scan_tmp = 0;
     size_t scan_tmp_elems = 0;
     uint32_t *u32_scratch = 0;   // small device counters
@@ -245,7 +249,6 @@ int k_unpack_particles(MpCtx* c, int n, float* pos3, float* vel3, int8_t* flag, 
                        float* T, float* L, float* sol, float* gas);
 int k_cells_to_startend(MpCtx* c, uint32_t* start, uint32_t* end);
 int k_phigra(MpCtx* c, float* ax, float* ay, float* az, const float* ls);
-int k_sweep_pass_swap(MpCtx* c, float** phi, int typeflag);
 int k_surface_tension_grid(MpCtx* c);
 int k_solid_phi(MpCtx* c);
 int k_delta_u(MpCtx* c);

@@ -390,8 +390,8 @@ __global__ void __launch_bounds__(256) k_ad_p2g_w(Grid g, const uint32_t* __rest
 // The same splat in FP32 with the engine's pair loop (p2g_walk): a column's
 // records fit one chunk, a lane's staging loads go out four at a time, and in
 // the air splat (PH 1) only the phase's records are staged. Per launch at 64^3
-// (dam) 225 -> DAM_P2G us, at 96^3 (column) water 1290 -> COL_P2GW us, air 770
-// -> COL_P2GA us against k_ad_p2g_w, which stays for FP64.
+// (dam) 225 -> 94 us, at 96^3 (column) water 1290 -> 585 us, air 770
+// -> 540 us against k_ad_p2g_w, which stays for FP64.
 template <int PH, int CAP>
 __global__ void __launch_bounds__(256, PH ? 3 : 2) k_ad_p2g_f(Grid g, const uint32_t* __restrict__ off,
                                                               const float4* __restrict__ xs4, const float4* __restrict__ vs4,
@@ -1099,7 +1099,7 @@ __global__ void k_ad_g2p_adj_p(Grid g, int np, const uint32_t* __restrict__ orde
 // each face, and its base and weights along k. A lane then only tests its k and
 // multiplies. Forming all of it in every lane took 105 instructions a candidate
 // (three divisions by h, three bases), this about 27: per launch at 64^3 (dam)
-// 1200 -> DAM_G2P us, at 96^3 (column) 1460 -> COL_G2P us.
+// 1200 -> 295 us, at 96^3 (column) 1460 -> 830 us.
 template <class T> struct G2pRec {   // one candidate; u/v: base along k and flags as bits
     alignas(16) T a[4];              // weight products of the x-, y- and z-face; base of the half coordinate | flags 28, 29
     alignas(16) T v[4];              // cotangent; base of the full coordinate | flag 28

@@ -223,15 +223,28 @@ __global__ void k_segsort(const uint32_t* __restrict__ off, int ncell, uint32_t*
 // each cell's type mask (which particle types it holds) from the particles'
 // type bytes in cell order (coalesced reads), and the bit of each brick (4^3
 // cells of the simulation grid, 8^3 of the 2x grid: bs = 2 or 3, as many bricks
-// on both) that holds an AIR or AIRSOLO particle
+// on both) that holds an AIR or AIRSOLO particle; with `bits` (the simulation
+// grid) also one bit per cell, by cell index, for AIR/AIRSOLO and, half_words
+// further, for FLUID/SOLID
 __global__ void k_tmask_sorted(const uint32_t* __restrict__ off, int ncell, int w, int hh, int d,
                                const uint8_t* __restrict__ types, uint8_t* __restrict__ tmask,
-                               uint32_t* __restrict__ air_words, int bs) {
-    MP_GRID_LOOP(cc, ncell) {
+                               uint32_t* __restrict__ air_words, int bs, uint32_t* __restrict__ bits, size_t half_words) {
+    // a warp-uniform loop: lane l of a warp holds cell c0 + l
+    const int lane = threadIdx.x & 31, stride = (int)(gridDim.x * blockDim.x);
+    for (int c0 = (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)); c0 < ncell; c0 += stride) {
+        const int cc = c0 + lane;
         uint32_t m = 0;
-        for (uint32_t s = off[cc]; s < off[cc + 1]; s++) m |= 1u << __ldg(types + s);
-        tmask[cc] = (uint8_t)m;
-        if ((m & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO)))) {
+        if (cc < ncell) {
+            for (uint32_t s = off[cc]; s < off[cc + 1]; s++) m |= 1u << __ldg(types + s);
+            tmask[cc] = (uint8_t)m;
+        }
+        const bool air = m & ((1u << MP_TYPEAIR) | (1u << MP_TYPEAIRSOLO));
+        if (bits) {
+            const unsigned wa = __ballot_sync(0xffffffffu, air);
+            const unsigned wf = __ballot_sync(0xffffffffu, (m & ((1u << MP_TYPEFLUID) | (1u << MP_TYPESOLID))) != 0);
+            if (lane == 0) { bits[c0 >> 5] = wa; bits[half_words + (c0 >> 5)] = wf; }
+        }
+        if (air) {
             const uint32_t kk = (uint32_t)cc % (uint32_t)d, jj = ((uint32_t)cc / (uint32_t)d) % (uint32_t)hh,
                            ii = (uint32_t)cc / ((uint32_t)d * (uint32_t)hh);
             const uint32_t up = (1u << bs) - 1, bw = ((uint32_t)d + up) >> bs, bh = ((uint32_t)hh + up) >> bs;
@@ -263,7 +276,8 @@ static int sort_on_grid(MpCtx* c, float dx, int w, int hh, int d) {
     MP_CUDA(c, cudaMemsetAsync(c->air_brick, 0, sizeof(uint32_t) * c->air_brick_words, c->stream));
     auto tmask_pass = [&](const uint8_t* types) -> int {
         k_tmask_sorted<<<mp_blocks(ncell, 256), 256, 0, c->stream>>>(c->cell_off, ncell, w, hh, d, types, c->tmask,
-                                                                     c->air_brick, sim_grid ? 2 : 3);
+                                                                     c->air_brick, sim_grid ? 2 : 3,
+                                                                     sim_grid ? c->cell_bits + 1 : nullptr, c->cell_bits_half);
         c->launches++;
         MP_CHECK_LAUNCH(c);
         return MP_OK;
