@@ -37,8 +37,8 @@ static void free_all(MpCtx* c) {
                     c->cell_tmp, c->mark, c->mark_tmp, c->cg_r, c->cg_p, c->cg_z, c->cg64, c->cg_exch, c->red, c->scal, c->red_count,
                     c->pos, c->vel, c->heat, c->pos2, c->vel2, c->heat2, c->pdens, c->pprs, c->pscr, c->pscr2,
                     c->flag_snap, c->pflag8, c->pflag8s, c->keys, c->perm, c->cell_cnt, c->cell_off, c->tmask, c->air_brick, c->cell_bits, c->scan_tmp, c->u32_scratch,
-                    c->randf, c->seeds, c->mc_numverts, c->mc_tri, c->mc_dens, c->mc_dens2, c->gfm_beta, c->gfm_s, c->mc_cube, c->mc_vflag, c->mc_vscan,
-                    c->mc_compact, c->mc_vverts, c->mc_vvscan, c->mc_emark, c->mc_escan, c->mc_vstart, c->mc_inc,
+                    c->randf, c->seeds, c->mc_numverts, c->mc_tri, c->mc_dens, c->mc_dens2, c->gfm_beta, c->gfm_s, c->mc_cube, c->mc_compact, c->mc_cbase,
+                    c->mc_rows, c->mc_first, c->mc_blocks, c->mc_escan, c->mc_edge_mask, c->mc_vstart, c->mc_inc,
                     c->mc_fill, c->mc_tmpv, c->pour_pos, c->pour_vel};
     k_adj_free(c);
     for (void* p : ptrs) if (p) cudaFree(p);
@@ -52,6 +52,23 @@ static void free_all(MpCtx* c) {
     for (int k = 0; k < MP_KT_COUNT; k++)
         for (auto& e : c->kt_pending[k]) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
+}
+
+// the cube's edges as corner pairs, corner v being bit v of the case index
+static const int kMcEdge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6},
+                                   {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
+// the edges that each case's triangles use; whether every case uses all that it crosses
+static int mc_edge_masks(const int32_t* nv, const int32_t* tri, uint32_t* masks) {
+    int complete = 1;
+    for (int cs = 0; cs < 256; cs++) {
+        uint32_t used = 0, crossed = 0;
+        for (int t = 0; t < nv[cs]; t++) used |= 1u << tri[cs * 16 + t];
+        for (int e = 0; e < 12; e++)
+            if (((cs >> kMcEdge[e][0]) & 1) != ((cs >> kMcEdge[e][1]) & 1)) crossed |= 1u << e;
+        masks[cs] = used;
+        if (used != crossed) complete = 0;
+    }
+    return complete;
 }
 
 static size_t scan_scratch(size_t n) {
@@ -134,18 +151,22 @@ static int create_impl(MpCtx* c, const mp_params* p) {
         mp_internal_mc_tables(nv, tri, nullptr);
         MP_CUDA(c, cudaMemcpy(c->mc_numverts, nv, sizeof(nv), cudaMemcpyHostToDevice));
         MP_CUDA(c, cudaMemcpy(c->mc_tri, tri, sizeof(tri), cudaMemcpyHostToDevice));
+        uint32_t masks[256];
+        c->mc_complete = mc_edge_masks(nv, tri, masks);
+        MP_TRY(dalloc_t(c, &c->mc_edge_mask, 256));
+        MP_CUDA(c, cudaMemcpy(c->mc_edge_mask, masks, sizeof(masks), cudaMemcpyHostToDevice));
     }
     size_t scan_max = std::max(kcap, n8 + 1);
     if (c->P.b_run_mc) {
         size_t nnode = (size_t)(2 * g.NX + 1) * (2 * g.NY + 1) * (2 * g.NZ + 1);
         size_t nvox = 8 * n;
-        c->mc_edges = 3 * nnode;
         MP_TRY(dalloc_t(c, &c->mc_dens, nnode)); MP_TRY(dalloc_t(c, &c->mc_dens2, nnode));
         MP_TRY(dalloc_t(c, &c->mc_cube, nvox));
-        MP_TRY(dalloc_t(c, &c->mc_vflag, nvox)); MP_TRY(dalloc_t(c, &c->mc_vscan, nvox + 1));
-        MP_TRY(dalloc_t(c, &c->mc_compact, nvox));
-        MP_TRY(dalloc_t(c, &c->mc_vverts, nvox)); MP_TRY(dalloc_t(c, &c->mc_vvscan, nvox + 1));
-        MP_TRY(dalloc_t(c, &c->mc_emark, c->mc_edges)); MP_TRY(dalloc_t(c, &c->mc_escan, c->mc_edges + 1));
+        MP_TRY(dalloc_t(c, &c->mc_compact, nvox)); MP_TRY(dalloc_t(c, &c->mc_cbase, nvox));
+        MP_TRY(dalloc_t(c, &c->mc_escan, 3 * nnode));
+        const size_t nrow = (size_t)(2 * g.NX + 1) * (2 * g.NY + 1);
+        MP_TRY(dalloc_t(c, &c->mc_rows, nrow)); MP_TRY(dalloc_t(c, &c->mc_first, nrow));
+        MP_TRY(dalloc_t(c, &c->mc_blocks, (nrow + 1023) / 1024));
         size_t mv = (size_t)c->P.mc_max_verts, mi = 3 * (size_t)c->P.mc_max_tris;
         MP_TRY(dalloc_t(c, &c->mc_vstart, mv + 1)); MP_TRY(dalloc_t(c, &c->mc_fill, mv + 1));
         MP_TRY(dalloc_t(c, &c->mc_inc, mi)); MP_TRY(dalloc_t(c, &c->mc_tmpv, mv));
@@ -153,7 +174,7 @@ static int create_impl(MpCtx* c, const mp_params* p) {
             MP_TRY(dalloc_t(c, &c->mc[a].verts, mv)); MP_TRY(dalloc_t(c, &c->mc[a].normals, mv));
             MP_TRY(dalloc_t(c, &c->mc[a].indices, mi));
         }
-        scan_max = std::max(scan_max, std::max(c->mc_edges + 1, mv + 1));
+        scan_max = std::max(scan_max, mv + 1);
     }
     c->scan_tmp_elems = scan_scratch(scan_max);
     MP_TRY(dalloc_t(c, &c->scan_tmp, c->scan_tmp_elems));
@@ -623,15 +644,12 @@ extern "C" int mp_mc_tables(int32_t* num_verts, int32_t* tri, int32_t* edge) {
 extern "C" int mp_set_mc_tables(void* ctx, const int32_t* num_verts, const int32_t* tri) {
     MpCtx* c = C(ctx); CTX_OR_ARG(c);
     if (!num_verts || !tri) { c->err = "set_mc_tables: null table"; return MP_ERR_ARG; }
-    // the cube's edges as corner pairs, corner v being bit v of the case index
-    static const int kEdge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6},
-                                     {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
     for (int cs = 0; cs < 256; cs++) {
         int nv = num_verts[cs];
         if (nv < 0 || nv > 15 || nv % 3) { c->err = "set_mc_tables: a vertex count is not 0..15 in steps of 3"; return MP_ERR_ARG; }
         for (int t = 0; t < nv; t++) {
             int e = tri[cs * 16 + t];
-            if (e < 0 || e > 11 || ((cs >> kEdge[e][0]) & 1) == ((cs >> kEdge[e][1]) & 1)) {
+            if (e < 0 || e > 11 || ((cs >> kMcEdge[e][0]) & 1) == ((cs >> kMcEdge[e][1]) & 1)) {
                 c->err = "set_mc_tables: a triangle uses an edge its case does not cross";
                 return MP_ERR_ARG;
             }
@@ -639,7 +657,11 @@ extern "C" int mp_set_mc_tables(void* ctx, const int32_t* num_verts, const int32
     }
     MP_CUDA(c, cudaMemcpyAsync(c->mc_numverts, num_verts, sizeof(int32_t) * 256, cudaMemcpyHostToDevice, c->stream));
     MP_CUDA(c, cudaMemcpyAsync(c->mc_tri, tri, sizeof(int32_t) * 256 * 16, cudaMemcpyHostToDevice, c->stream));
+    uint32_t masks[256];
+    const int complete = mc_edge_masks(num_verts, tri, masks);
+    MP_CUDA(c, cudaMemcpyAsync(c->mc_edge_mask, masks, sizeof(masks), cudaMemcpyHostToDevice, c->stream));
     MP_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->mc_complete = complete;
     return MP_OK;
 }
 
@@ -1070,7 +1092,7 @@ extern "C" int mp_step(void* ctx) {
     if (P.b_run_mc && P.mc_every > 0 && c->S.frame % P.mc_every == 0) {
         MP_STAGE("preMC", k_mc_presort(c));
         if (kept_solid) MP_STAGE("runMC_interaction", k_mc_renormal(c, MP_MC_SOLID));
-        else MP_STAGE("runMC_smooth", k_mc(c, MP_MC_SOLID));
+        else MP_STAGE("runMC_smooth", k_mc(c, MP_MC_SOLID, false));
         MP_STAGE("runMC_fluid_gas", k_mc_fluid_gas(c));
     }
     // a file that cannot be written ends the step's output, not the step

@@ -107,11 +107,13 @@ struct MpCtx {
     float *mc_dens2 = 0;              // gas field of the fused fluid+gas density pass
     const float* mc_last_dens = 0;    // field of the last extraction
     uint8_t *mc_cube = 0;
-    uint32_t *mc_vflag = 0, *mc_vscan = 0, *mc_compact = 0, *mc_vverts = 0, *mc_vvscan = 0;
-    uint32_t *mc_emark = 0, *mc_escan = 0;
+    uint32_t *mc_compact = 0, *mc_cbase = 0;   // active voxels and their first index
+    uint4 *mc_rows = 0, *mc_first = 0, *mc_blocks = 0;   // per row of nodes: counts, their scan
+    uint32_t *mc_escan = 0;           // vertex of each crossed edge
+    uint32_t *mc_edge_mask = 0;       // edges that each case's triangles use
+    int mc_complete = 1;              // every case uses all edges that it crosses
     uint32_t *mc_vstart = 0, *mc_inc = 0, *mc_fill = 0;
     float3 *mc_tmpv = 0;
-    size_t mc_edges = 0;
     int mc_sorted = 0;           // particles currently sorted on the 2x grid
     McSurface mc[3];
     int mc_cap_verts = 0, mc_cap_idx = 0;
@@ -222,7 +224,7 @@ int k_gen_gas(MpCtx* c);
 int k_delete(MpCtx* c);
 int k_melt(MpCtx* c);
 int k_freeze(MpCtx* c);
-int k_mc(MpCtx* c, int surface);
+int k_mc(MpCtx* c, int surface, bool keep_field = true);
 int k_mc_fluid_gas(MpCtx* c);
 int k_cg_res_setup(MpCtx* c);
 int k_cg_solve(MpCtx* c, const int8_t* mark, float* x, const float* b, int maxiter, int tolmode, float tol, int* iters,
