@@ -29,6 +29,7 @@ struct ResGeom {
 struct ResPlan {
     ResGeom g{};
     int nblk = 0, Q = 0;
+    bool one = false;   // one exchange an iteration (FP32)
     size_t smem = 0;
 };
 

@@ -905,8 +905,9 @@ int k_cg_res_setup(MpCtx* c) {
     MP_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
     if (!coop || !c->cg_use_res) return MP_OK;
     const size_t room = (size_t)smem - 1024;   // the kernel's static shared memory
-    c->res_plan32 = res_plan<float>(c->G, sms, room);
-    c->res_plan64 = res_plan<double>(c->G, sms, room);
+    c->res_plan32 = res_plan<float>(c->G, sms, room, true);
+    if (!c->res_plan32.nblk || c->res_plan32.Q > RES_ONE_Q) c->res_plan32 = res_plan<float>(c->G, sms, room, false);
+    c->res_plan64 = res_plan<double>(c->G, sms, room, false);
     const size_t words = std::max(c->res_plan32.nblk ? res_exch_words(c->res_plan32) : 0,
                                   c->res_plan64.nblk ? res_exch_words(c->res_plan64) : 0);
     if (!words) return MP_OK;
@@ -924,18 +925,31 @@ static int run_cg_res(MpCtx* c, const Op& op, R* x, const R* b, int maxiter, int
     *taken = P.nblk > 0 && maxiter < (1 << 28);
     if (!*taken) return MP_OK;
     void (*kern)(Op, ResGeom, const R*, R*, uint64_t*, uint64_t*, Red, int, float, int, uint32_t) = nullptr;
-    switch (P.Q) {
-    case 1: kern = k_cg_res<R, Op, 1>; break;
-    case 2: kern = k_cg_res<R, Op, 2>; break;
-    case 3: kern = k_cg_res<R, Op, 3>; break;
-    case 4: kern = k_cg_res<R, Op, 4>; break;
-    case 6: kern = k_cg_res<R, Op, 6>; break;
-    default: kern = k_cg_res<R, Op, 8>;
+    if constexpr (sizeof(R) == 4) {
+        if (P.one) {
+            switch (P.Q) {
+            case 1: kern = k_cg_res<R, Op, 1, true>; break;
+            case 2: kern = k_cg_res<R, Op, 2, true>; break;
+            case 3: kern = k_cg_res<R, Op, 3, true>; break;
+            default: kern = k_cg_res<R, Op, 4, true>;
+            }
+        } else {
+            kern = P.Q <= 6 ? k_cg_res<R, Op, 6, false> : k_cg_res<R, Op, 8, false>;
+        }
+    } else {
+        switch (P.Q) {
+        case 1: kern = k_cg_res<R, Op, 1, false>; break;
+        case 2: kern = k_cg_res<R, Op, 2, false>; break;
+        case 3: kern = k_cg_res<R, Op, 3, false>; break;
+        case 4: kern = k_cg_res<R, Op, 4, false>; break;
+        case 6: kern = k_cg_res<R, Op, 6, false>; break;
+        default: kern = k_cg_res<R, Op, 8, false>;
+        }
     }
     cudaStream_t s = c->stream;
     Red Rd = red_of(c);
     // tags run on from solve to solve; start over before they could wrap
-    if (c->cg_epoch > 0xffffffffu - 2u * (uint32_t)std::max(maxiter, 0) - 4u) {
+    if (c->cg_epoch > 0xffffffffu - 2u * (uint32_t)std::max(maxiter, 0) - 8u) {
         MP_CUDA(c, cudaMemsetAsync(c->cg_exch, 0, sizeof(uint64_t) * c->cg_exch_words, s));
         c->cg_epoch = 1;
     }
@@ -963,7 +977,7 @@ static int run_cg_res(MpCtx* c, const Op& op, R* x, const R* b, int maxiter, int
         c->err = "cg: an exchange between thread blocks ran out of time";
         return MP_ERR_TIMEOUT;
     }
-    c->cg_epoch += 2u * hflag[F_ITERS] + 4u;
+    c->cg_epoch += 2u * hflag[F_ITERS] + 8u;
     *iters_out = (int)hflag[F_ITERS];
     *res_out = rr;
     c->work[MP_WC_CG_ITERS] += hflag[F_ITERS];
