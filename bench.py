@@ -32,20 +32,17 @@ CG_UPD_BYTES_PER_CELL = 21
 
 def names_kt(mp):
     return {mp.KT_CG_STENCIL: "k_cg_dir", mp.KT_CG_UPDATE: "k_cg_upd", mp.KT_P2G: "k_p2g",
-            mp.KT_G2P: "k_g2p", mp.KT_SORT: "sort", mp.KT_LEVELSET: "k_genlevelset", mp.KT_MC_DENS: "k_mc_density",
-            mp.KT_CORRECT: "k_correct_pos"}
+            mp.KT_G2P: "k_g2p", mp.KT_SORT: "sort", mp.KT_LEVELSET: "k_genlevelset", mp.KT_MC_DENS: "k_mc_pairs",
+            mp.KT_CORRECT: "k_correct_springs"}
 
 
 # DRAM bytes per launch from ncu captures (dram__bytes_read.sum + dram__bytes_write.sum),
 # as functions of (cells, particles): the capture's bytes scaled by the units a
 # launch processes
 TRAFFIC_PER_LAUNCH = {
-    # the TMA CG passes captured at 256^3: 189.4 MB and 294.5 MB per launch
-    "k_cg_dir": lambda n, np_: 189.36e6 * n / 256 ** 3,
-    "k_cg_upd": lambda n, np_: 294.46e6 * n / 256 ** 3,
-    # the MC density pass captured at 128^3 (12.9M particles): 711.9 MB per
-    # launch; nodes and particles both grow with the cells
-    "k_mc_density": lambda n, np_: 711.91e6 * n / 128 ** 3,
+    # the TMA CG passes captured at 224^3 (--profile-case cg): 120.6 MB and 174.1 MB per launch
+    "k_cg_dir": lambda n, np_: 120.59e6 * n / 224 ** 3,
+    "k_cg_upd": lambda n, np_: 174.06e6 * n / 224 ** 3,
 }
 
 
@@ -256,8 +253,12 @@ def profile_case(args):
         out = {"case": "cg", "n": n, "iterations": it, "rc": rc, "solve_ms": (time.perf_counter() - t0) * 1e3}
         for k, (nm, bpc) in classes.items():
             ms, nl = sim.kernel_timing_read(k)
-            per = ms / max(nl, 1)
+            if nl == 0:
+                continue
+            per = ms / nl
             out[nm] = {"launches": nl, "us_per_launch": per * 1e3, "algorithmic_GBps": bpc * n ** 3 / (per / 1e3) / 1e9}
+        if nl == 0:   # the whole solve is one launch (grids that fit on chip)
+            out["k_cg_res"] = {"launches": out["k_cg_dir"]["launches"], "ms": out.pop("k_cg_dir")["us_per_launch"] / 1e3}
     else:
         sim = mp.Sim.from_config(args.config, n, args.seed)
         sim.bubblesim()
@@ -570,17 +571,17 @@ def main():
                                 CG_DIR_BYTES_PER_CELL * n * wc["cg_iters"], wc["cg_iters"]),
              mp.KT_CG_UPDATE: ("k_cg_tma<PressOp,1> (A p, x and r update, r.r)",
                                CG_UPD_BYTES_PER_CELL * n * wc["cg_iters"], wc["cg_iters"]),
-             mp.KT_P2G: ("k_p2g_water + k_p2g_air (water + air launches)", (29 * npart + 56 * n) * kt[mp.KT_P2G][1],
+             mp.KT_P2G: ("k_p2g_staged (water + air launches)", (29 * npart + 56 * n) * kt[mp.KT_P2G][1],
                          kt[mp.KT_P2G][1]),
              mp.KT_G2P: ("k_g2p", (37 * npart + 72 * n) * kt[mp.KT_G2P][1], kt[mp.KT_G2P][1]),
              mp.KT_SORT: ("hash sort (count, scan, scatter, segment sort, gather)",
                           (102 * npart + 8 * n) * wc["sort_full"] + (12 * npart + 8 * n) * wc["sort_fast"],
                           wc["sort_full"] + wc["sort_fast"]),
              mp.KT_LEVELSET: ("k_genlevelset", (13 * npart + 9 * n) * kt[mp.KT_LEVELSET][1], kt[mp.KT_LEVELSET][1]),
-             mp.KT_MC_DENS: ("k_mc_density (fused fluid + gas fields at 2x)", (13 * npart + 64 * n) * kt[mp.KT_MC_DENS][1],
+             mp.KT_MC_DENS: ("k_mc_pairs (fused fluid + gas fields at 2x)", (13 * npart + 64 * n) * kt[mp.KT_MC_DENS][1],
                              kt[mp.KT_MC_DENS][1]),
              # read each position record and neighbour mass, write the corrected record; cell ranges
-             mp.KT_CORRECT: ("k_correct_pos (particle spacing spring)", (36 * npart + 4 * n) * kt[mp.KT_CORRECT][1],
+             mp.KT_CORRECT: ("k_correct_springs (particle spacing spring)", (36 * npart + 4 * n) * kt[mp.KT_CORRECT][1],
                              kt[mp.KT_CORRECT][1])}
     dom = max(model, key=lambda k: kt[k][0])
     ms_k = kt[dom][0]

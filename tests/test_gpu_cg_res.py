@@ -66,6 +66,19 @@ def test_on_chip_solve_equals_the_passes(mp, monkeypatch, shape, form):
         assert b[4] < 8, b[4]
 
 
+# the TMA passes by name (grids of these sizes take the on-chip solve): partial
+# tiles along j and k, one plane chunk and many, a row of one group
+@pytest.mark.parametrize("shape", [(40, 24, 48), (64, 64, 64), (9, 17, 16), (170, 20, 80)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_tma_passes_equal_the_float4_passes(mp, monkeypatch, shape):
+    a = _project(mp, monkeypatch, "v4", shape, mp.PREC_MIXED, 1e-6)
+    b = _project(mp, monkeypatch, "tma", shape, mp.PREC_MIXED, 1e-6)
+    assert a[1] == b[1] == 0
+    assert abs(a[0] - b[0]) <= 1, (a[0], b[0])
+    assert rel_err(b[2], a[2]) <= 1e-5 and rel_err(b[3], a[3]) <= 1e-5
+    assert b[4] > 8, b[4]
+
+
 def test_iteration_cap_and_empty_right_hand_side(mp, monkeypatch):
     """The cap stops after exactly that many iterations with the warning code;
     a zero right-hand side needs none."""
