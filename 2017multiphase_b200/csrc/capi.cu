@@ -318,6 +318,7 @@ extern "C" int mp_upload_particles(void* ctx, int n, const float* pos3, const fl
     MP_CUDA(c, cudaStreamSynchronize(c->stream));
     c->S.par_num_now = n;
     c->mc_sorted = 0;
+    c->types_stale = true;
     return MP_OK;
 }
 extern "C" int mp_download_particles(void* ctx, int* n, float* pos3, float* vel3, int8_t* flag, float* mass,
@@ -462,6 +463,7 @@ extern "C" int mp_set_field(void* ctx, int f, const void* src, size_t bytes) {
         }
         memcpy(dstp, src, bytes);
         MP_TRY(k_pack_particles(c, np, p3.data(), v3.data(), fl.data(), m.data(), T.data(), L.data(), so.data(), ga.data()));
+        if (f == MP_P_FLAG) c->types_stale = true;
     } else {
         void* d = field_dev(c, f, cnt, e);
         MP_CUDA(c, cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, c->stream));
@@ -633,6 +635,7 @@ extern "C" int mp_checkpoint_load(void* ctx, const void* host_src, size_t bytes)
     MP_CUDA(c, cudaStreamSynchronize(s));
     c->S = h.state;
     c->mc_sorted = 0;
+    c->types_stale = true;
     return MP_OK;
 }
 
@@ -736,7 +739,7 @@ extern "C" int64_t mp_launch_count(void* ctx) {
 // ---------------------------------------------------------------------------
 static int need_cells(MpCtx* c) {
     if (c->mc_sorted) { c->err = "particles are sorted on the marching-cubes grid; call mp_hash_sort first"; return MP_ERR_STATE; }
-    return MP_OK;
+    return k_refresh_types(c);
 }
 #define STAGE(name, body)                                  \
     extern "C" int name(void* ctx) {                       \
@@ -792,6 +795,7 @@ extern "C" int mp_mc(void* ctx, int surface) {
     MpCtx* c = C(ctx); CTX_OR_ARG(c);
     if (surface < 0 || surface > 2) return MP_ERR_ARG;
     if (!c->P.b_run_mc) { c->err = "marching cubes disabled at mp_create"; return MP_ERR_STATE; }
+    if (c->mc_sorted) MP_TRY(k_refresh_types(c));
     return k_mc(c, surface);
 }
 extern "C" int mp_mc_download(void* ctx, int surface, float* verts, float* normals, uint32_t* indices, int max_verts,

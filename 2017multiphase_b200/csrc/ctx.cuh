@@ -95,6 +95,10 @@ struct MpCtx {
     // after: AIR/AIRSOLO, then FLUID/SOLID cell_bits_half words further
     uint32_t *cell_bits = 0;
     size_t cell_bits_half = 0;
+    // the last sort: its particle count and grid; whether particles have been
+    // replaced since, so that the masks, bricks and bits are the old types'
+    int sorted_np = 0;
+    bool sorted_2x = false, types_stale = false;
     uint32_t *scan_tmp = 0;
     size_t scan_tmp_elems = 0;
     uint32_t *u32_scratch = 0;   // small device counters
@@ -193,6 +197,7 @@ struct KtScope {
 int mp_scan_u32(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n);   // exclusive scan, out[n] = total
 int k_hash_sort(MpCtx* c);
 int k_mc_presort(MpCtx* c);
+int k_refresh_types(MpCtx* c);
 int k_external_force(MpCtx* c);
 int k_levelset(MpCtx* c);
 int k_sweep_ls_mark(MpCtx* c);

@@ -1225,6 +1225,7 @@ int k_delete(MpCtx* c) {
     MP_CUDA(c, cudaStreamSynchronize(c->stream));
     std::swap(c->pos, c->pos2); std::swap(c->vel, c->vel2); std::swap(c->heat, c->heat2);
     c->S.par_num_now = (int)total;
+    if ((int)total != np) c->types_stale = true;   // other particles in the cells' ranges
     return MP_OK;
 }
 

@@ -253,6 +253,9 @@ __global__ void k_tmask_sorted(const uint32_t* __restrict__ off, int ncell, int 
         }
     }
 }
+__global__ void k_types(int np, const float4* __restrict__ pos, uint8_t* __restrict__ types) {
+    MP_GRID_LOOP(p, np) types[p] = (uint8_t)(pflag(pos[p]) & 7);
+}
 __global__ void k_reorder(const uint32_t* __restrict__ perm, int np,
                           const float4* __restrict__ p0, const float4* __restrict__ v0, const float4* __restrict__ h0,
                           float4* __restrict__ p1, float4* __restrict__ v1, float4* __restrict__ h1,
@@ -267,21 +270,40 @@ __global__ void k_reorder(const uint32_t* __restrict__ perm, int np,
 }
 }  // namespace
 
-static int sort_on_grid(MpCtx* c, float dx, int w, int hh, int d) {
+// the cells' type masks, brick map and cell bits from the types of the particles
+// in sorted order
+static int cell_types(MpCtx* c, const uint8_t* types, bool grid2x) {
+    const int f = grid2x ? 2 : 1, w = f * c->G.NX, hh = f * c->G.NY, d = f * c->G.NZ, ncell = w * hh * d;
+    MP_CUDA(c, cudaMemsetAsync(c->air_brick, 0, sizeof(uint32_t) * c->air_brick_words, c->stream));
+    k_tmask_sorted<<<mp_blocks(ncell, 256), 256, 0, c->stream>>>(c->cell_off, ncell, w, hh, d, types, c->tmask,
+                                                                 c->air_brick, grid2x ? 3 : 2,
+                                                                 grid2x ? nullptr : c->cell_bits + 1, c->cell_bits_half);
+    c->launches++;
+    MP_CHECK_LAUNCH(c);
+    return MP_OK;
+}
+// The same after particles have been replaced (types_stale) and before the next
+// sort: the stages then read the new types in the last sort's ranges, and a cell
+// whose mask were still the old particles' would be passed over.
+int k_refresh_types(MpCtx* c) {
+    if (!c->types_stale) return MP_OK;
+    c->types_stale = false;
+    if (c->sorted_np <= 0) return MP_OK;
+    k_types<<<mp_blocks(c->sorted_np, 256), 256, 0, c->stream>>>(c->sorted_np, c->pos, c->pflag8);
+    c->launches++;
+    MP_CHECK_LAUNCH(c);
+    return cell_types(c, c->pflag8, c->sorted_2x);
+}
+
+static int sort_on_grid(MpCtx* c, float dx, bool grid2x) {
+    const int f = grid2x ? 2 : 1, w = f * c->G.NX, hh = f * c->G.NY, d = f * c->G.NZ;
     int np = c->np();
     int ncell = w * hh * d;
     uint32_t* unsorted = c->u32_scratch + 1;
     MP_CUDA(c, cudaMemsetAsync(unsorted, 0, sizeof(uint32_t), c->stream));
-    const bool sim_grid = w == c->G.NX && hh == c->G.NY && d == c->G.NZ;
-    MP_CUDA(c, cudaMemsetAsync(c->air_brick, 0, sizeof(uint32_t) * c->air_brick_words, c->stream));
-    auto tmask_pass = [&](const uint8_t* types) -> int {
-        k_tmask_sorted<<<mp_blocks(ncell, 256), 256, 0, c->stream>>>(c->cell_off, ncell, w, hh, d, types, c->tmask,
-                                                                     c->air_brick, sim_grid ? 2 : 3,
-                                                                     sim_grid ? c->cell_bits + 1 : nullptr, c->cell_bits_half);
-        c->launches++;
-        MP_CHECK_LAUNCH(c);
-        return MP_OK;
-    };
+    c->types_stale = false;
+    c->sorted_np = np;
+    c->sorted_2x = grid2x;
     if (np > 0) {
         k_hash_count<<<mp_blocks(np, 256), 256, 0, c->stream>>>(c->pos, np, c->G.gx0, c->G.gy0, c->G.gz0, dx, w, hh, d,
                                                                 c->keys, c->cell_cnt, unsorted, c->pflag8);
@@ -297,7 +319,7 @@ static int sort_on_grid(MpCtx* c, float dx, int w, int hh, int d) {
         // already in cell order: the stable sort is the identity permutation;
         // the counts still have to run back to zero for the next sort
         MP_CUDA(c, cudaMemsetAsync(c->cell_cnt, 0, sizeof(uint32_t) * ncell, c->stream));
-        return tmask_pass(c->pflag8);
+        return cell_types(c, c->pflag8, grid2x);
     }
     if (np > 0) {
         k_scatter<<<mp_blocks(np, 256), 256, 0, c->stream>>>(c->keys, np, c->cell_off, c->cell_cnt, c->perm);
@@ -314,22 +336,21 @@ static int sort_on_grid(MpCtx* c, float dx, int w, int hh, int d) {
         MP_CHECK_LAUNCH(c);
         std::swap(c->pos, c->pos2); std::swap(c->vel, c->vel2); std::swap(c->heat, c->heat2);
     }
-    return tmask_pass(np > 0 ? c->pflag8s : c->pflag8);
+    return cell_types(c, np > 0 ? c->pflag8s : c->pflag8, grid2x);
 }
 
 int k_hash_sort(MpCtx* c) {
     KtScope kt(c, MP_KT_SORT);
     c->mc_sorted = 0;
-    return sort_on_grid(c, c->G.h, c->G.NX, c->G.NY, c->G.NZ);
+    return sort_on_grid(c, c->G.h, false);
 }
 
 // preMC + hashAndSortParticles_MC (spray.cu:759-765, 639-662): cell size
 // cellsize/NXMC*NX on the 2x grid (calcHashD_MC, spray_k.cu:1030-1048)
 int k_mc_presort(MpCtx* c) {
     KtScope kt(c, MP_KT_SORT);
-    int NXMC = 2 * c->G.NX, NYMC = 2 * c->G.NY, NZMC = 2 * c->G.NZ;
-    float dx = c->G.h / (float)NXMC * (float)c->G.NX;
-    MP_TRY(sort_on_grid(c, dx, NXMC, NYMC, NZMC));
+    float dx = c->G.h / (float)(2 * c->G.NX) * (float)c->G.NX;
+    MP_TRY(sort_on_grid(c, dx, true));
     c->mc_sorted = 1;
     return MP_OK;
 }
