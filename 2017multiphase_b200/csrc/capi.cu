@@ -318,7 +318,7 @@ extern "C" int mp_upload_particles(void* ctx, int n, const float* pos3, const fl
     MP_CUDA(c, cudaStreamSynchronize(c->stream));
     c->S.par_num_now = n;
     c->mc_sorted = 0;
-    c->types_stale = true;
+    c->types_stale = c->moved = true;
     return MP_OK;
 }
 extern "C" int mp_download_particles(void* ctx, int* n, float* pos3, float* vel3, int8_t* flag, float* mass,
@@ -464,6 +464,7 @@ extern "C" int mp_set_field(void* ctx, int f, const void* src, size_t bytes) {
         memcpy(dstp, src, bytes);
         MP_TRY(k_pack_particles(c, np, p3.data(), v3.data(), fl.data(), m.data(), T.data(), L.data(), so.data(), ga.data()));
         if (f == MP_P_FLAG) c->types_stale = true;
+        if (f == MP_P_POS) c->moved = true;
     } else {
         void* d = field_dev(c, f, cnt, e);
         MP_CUDA(c, cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, c->stream));
@@ -635,7 +636,7 @@ extern "C" int mp_checkpoint_load(void* ctx, const void* host_src, size_t bytes)
     MP_CUDA(c, cudaStreamSynchronize(s));
     c->S = h.state;
     c->mc_sorted = 0;
-    c->types_stale = true;
+    c->types_stale = c->moved = true;
     return MP_OK;
 }
 

@@ -95,10 +95,12 @@ struct MpCtx {
     // after: AIR/AIRSOLO, then FLUID/SOLID cell_bits_half words further
     uint32_t *cell_bits = 0;
     size_t cell_bits_half = 0;
-    // the last sort: its particle count and grid; whether particles have been
-    // replaced since, so that the masks, bricks and bits are the old types'
+    // the last sort: its particle count, the cells that hold any, its grid; whether
+    // particles have been replaced since, so that the masks, bricks and bits are
+    // the old types', and whether any may have moved
     int sorted_np = 0;
-    bool sorted_2x = false, types_stale = false;
+    uint32_t sorted_cells = 0;
+    bool sorted_2x = false, types_stale = false, moved = true;
     uint32_t *scan_tmp = 0;
     size_t scan_tmp_elems = 0;
     uint32_t *u32_scratch = 0;   // small device counters
@@ -194,7 +196,8 @@ struct KtScope {
 };
 
 // stage entry points implemented across the kernel files
-int mp_scan_u32(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n);   // exclusive scan, out[n] = total
+// exclusive scan, out[n] = total; nonzero: the entries that are not 0 are counted into it
+int mp_scan_u32(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n, uint32_t* nonzero = nullptr);
 int k_hash_sort(MpCtx* c);
 int k_mc_presort(MpCtx* c);
 int k_refresh_types(MpCtx* c);

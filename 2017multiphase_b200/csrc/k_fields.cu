@@ -606,8 +606,8 @@ int k_surface_tension_grid(MpCtx* c) {
 }
 
 int k_solid_phi(MpCtx* c) {
-    MP_CUDA(c, cudaMemsetAsync(c->u32_scratch + 2, 0, sizeof(uint32_t), c->stream));
-    k_init_solid_phi<<<mp_blocks(c->G.n, 256), 256, 0, c->stream>>>(c->G, cells_of(c), c->phisolid, c->u32_scratch + 2);
+    MP_CUDA(c, cudaMemsetAsync(c->u32_scratch + 6, 0, sizeof(uint32_t), c->stream));
+    k_init_solid_phi<<<mp_blocks(c->G.n, 256), 256, 0, c->stream>>>(c->G, cells_of(c), c->phisolid, c->u32_scratch + 6);
     c->launches++;
     MP_CHECK_LAUNCH(c);
     return sweep_one(c, &c->phisolid, nullptr, -1, 3);

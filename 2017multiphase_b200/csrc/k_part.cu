@@ -289,21 +289,133 @@ __global__ void k_collide_freezing(Grid g, Cells cl, int np, const float4* __res
     }
 }
 
-// correctparticlepos: reads pos, writes out (out of place)
+// correctparticlepos: reads pos, writes out (out of place), in two kernels.
 //
+// The cells that a particle's pairs can lie in, as a range of columns and the k
+// range of each.
+struct CpWindow {
+    int i, j, k, ilo, ihi, jlo, jhi, k0, k1;
+    __device__ __forceinline__ CpWindow(const Grid& g, float3 ip, float re) {
+        const float h = g.h;
+        ijkpos(g, ip, i, j, k);
+        // With re below half a cell, a neighbour cell on the far side of the
+        // particle's own half-cell holds only particles whose d2 exceeds
+        // 1.001 re^2 (its whole extent is more than 1.002 re away along that
+        // axis, with a margin for the rounding of the cell coordinates), so
+        // every pair in it would be skipped: the cell is not visited.
+        const float3 rel = (ip - mk3(g.gx0, g.gy0, g.gz0)) / mk3(h, h, h);
+        const float cut_lo = 1.002f * (re / h) + 2e-4f;
+        auto span = [&](float r, int n, int c, int& lo, int& hi) {
+            lo = -1; hi = 1;
+            if (r >= 0 && r < (float)n) {
+                float fr = r - (float)c;
+                if (fr > cut_lo) lo = 0;
+                if (1.0f - fr > cut_lo) hi = 0;
+            }
+        };
+        int klo, khi;
+        span(rel.x, g.NX, i, ilo, ihi); span(rel.y, g.NY, j, jlo, jhi); span(rel.z, g.NZ, k, klo, khi);
+        // columns outside the grid fall away
+        ilo = max(ilo, -i); ihi = min(ihi, g.NX - 1 - i);
+        jlo = max(jlo, -j); jhi = min(jhi, g.NY - 1 - j);
+        k0 = max(k + klo, 0); k1 = min(k + khi, g.NZ - 1);
+    }
+    // the cells of a (di,dj) column are contiguous: the bounds of up to three of
+    // them, read together (those beyond k1 are empty)
+    __device__ __forceinline__ void bounds(const Grid& g, const Cells& cl, int di, int dj, uint32_t (&bnd)[4]) const {
+        const int cb = cid(g, i + di, j + dj, k0);
+        #pragma unroll
+        for (int u = 0; u < 4; u++) bnd[u] = __ldg(cl.off + cb + min(u, k1 - k0 + 1));
+    }
+};
+// the particle at ip moved by its springs' sum
+__device__ __forceinline__ float3 cp_moved(const Grid& g, float3 ip, float3 spring, float re, float spring_k, float samplespace,
+                                           float dt) {
+    const float h = g.h;
+    const float3 g0 = mk3(g.gx0, g.gy0, g.gz0);
+    const float3 g1 = g0 + mk3((float)g.NX, (float)g.NY, (float)g.NZ) * h;
+    const float3 tmin = g0 + (mk3(h, h, h) + mk3(0.5f * samplespace));
+    const float3 tmax = g1 - (mk3(h, h, h) + mk3(0.5f * samplespace));
+    spring *= spring_k * re;
+    if (length(dt * spring) > 0.3f * h) ip += h * 0.3f * spring / length(spring);
+    else ip += dt * spring;
+    return mk3(fmaxf(tmin.x, fminf(tmax.x, ip.x)), fmaxf(tmin.y, fminf(tmax.y, ip.y)), fmaxf(tmin.z, fminf(tmax.z, ip.z)));
+}
+// Two phases keep a warp's lanes together: the scan collects the pairs within re
+// (a few of the candidates) in visiting order, marked where a new cell starts;
+// the spring terms of the collected pairs are then formed in that order, each
+// cell's sum added to the total when the next cell starts (a cell without pairs
+// adds +0, a no-op). A full buffer is drained in the middle of the scan. Beyond re
+// the kernel weight is exactly zero and the pair adds a signed zero, which leaves
+// the sum unchanged: it is skipped (exact test with margin: dist*dist >= re*re
+// whenever d2 > 1.001 re*re).
+struct CpSum {
+    float3 spring = mk3(0.0f), cell = mk3(0.0f);
+    __device__ __forceinline__ void pair(float3 ip, float3 o, float m, float re, bool first) {
+        if (first) { spring += cell; cell = mk3(0.0f); }
+        const float3 dd = o - ip;
+        const float dist = length(dd);
+        const float w = m * smooth_kernel(dist * dist, re);
+        if (dist > 0.1f * re) cell += w * (ip - o) / dist;
+    }
+};
+constexpr int CP_BUF = 16;
+
+// One thread a particle, candidates from global memory through L1, which is all
+// this kernel's: for particles that are sparse, or no longer in sorted order.
+__global__ void __launch_bounds__(256, 6) k_correct_gather(Grid g, Cells cl, int np, const float4* __restrict__ pos,
+                                                           const float4* __restrict__ vel, float4* __restrict__ out, float re,
+                                                           float spring_k, float samplespace, float dt) {
+    const float re2_skip = re * re * 1.001f;
+    MP_GRID_LOOP(p, np) {
+        const float4 q = pos[p];
+        const int f = pflag(q);
+        if (f == MP_TYPESOLID || f == MP_TYPEAIRSOLO) { out[p] = q; continue; }
+        const float3 ip = xyz(q);
+        const CpWindow W(g, ip, re);
+        uint32_t ent[CP_BUF];   // | 1 << 31: the first of its cell
+        int ne = 0;
+        CpSum S;
+        auto drain = [&]() {
+            for (int e = 0; e < ne; e++) {
+                const uint32_t t = ent[e] & 0x7fffffffu;
+                S.pair(ip, xyz(__ldg(pos + t)), __ldg(&vel[t].w), re, ent[e] >> 31);
+            }
+            ne = 0;
+        };
+        for (int di = W.ilo; di <= W.ihi; di++) for (int dj = W.jlo; dj <= W.jhi; dj++) {
+            uint32_t bnd[4];
+            W.bounds(g, cl, di, dj, bnd);
+            for (int cc = 0; cc <= W.k1 - W.k0; cc++) {
+                uint32_t first = 0x80000000u;
+                for (uint32_t t = bnd[cc]; t < bnd[cc + 1]; ++t) {
+                    const float3 dd = xyz(__ldg(pos + t)) - ip;
+                    if (dot(dd, dd) > re2_skip) continue;
+                    if (ne == CP_BUF) drain();
+                    ent[ne++] = t | first;
+                    first = 0;
+                }
+            }
+        }
+        drain();
+        out[p] = with_xyz(q, cp_moved(g, ip, S.spring + S.cell, re, spring_k, samplespace, dt));
+    }
+}
+
 // A block's particles, consecutive in the sorted order, lie in consecutive cells
 // cA .. cB; shifted by a neighbour column (di, dj) those cells, and one more at
 // either end, are again consecutive and so is the particle range that they hold.
 // The block copies these nine ranges (position and mass) into shared memory with
 // coalesced loads and every lane walks its own cells there. When they do not all
-// fit, they go in batches of whole columns in visiting order; a column that
-// alone exceeds CAP is read from global memory. Candidates are tested two to an
-// instruction into a bit mask, so the scan has no branch per candidate.
+// fit, they go in batches of whole columns in visiting order; where a column
+// alone exceeds CAP, the block reads its candidates from global memory. Candidates
+// are tested two to an instruction into a bit mask, so the scan has no branch per
+// candidate.
 // One gather per candidate and lane from global memory kept L1 at its limit (79 %).
-// 256^3 bubble column: 19.7 -> 18.1 ms; 32^3: 49 -> 37 us. What is left is the
-// latency of the collected pairs' square root and divisions: neither more
-// resident warps (64, 72 or 80 registers) nor wider shared loads changed it.
-constexpr int CP_T = 128, CP_CAP = 1472, CP_BUF = 16;
+// What is left is the latency of the collected pairs' square root and divisions:
+// neither more resident warps (64, 72 or 80 registers) nor wider shared loads
+// changed it.
+constexpr int CP_T = 128, CP_CAP = 1472;
 constexpr int CP_ROW = CP_CAP + 8;   // a group of 8 candidates may start on the last one
 constexpr int CP_SMEM = 4 * CP_ROW * (int)sizeof(float) + CP_BUF * CP_T * (int)sizeof(uint16_t);
 __global__ void __launch_bounds__(CP_T, 8) k_correct_springs(Grid g, Cells cl, int np, const float4* __restrict__ pos, const float4* __restrict__ vel,
@@ -312,14 +424,9 @@ __global__ void __launch_bounds__(CP_T, 8) k_correct_springs(Grid g, Cells cl, i
     float* const sx = reinterpret_cast<float*>(cp_st);
     float *const sy = sx + CP_ROW, *const sz = sy + CP_ROW, *const sm = sz + CP_ROW;
     uint16_t* const hits16 = reinterpret_cast<uint16_t*>(sm + CP_ROW) + threadIdx.x;
-    uint32_t* const hits32 = reinterpret_cast<uint32_t*>(sm + CP_ROW) + threadIdx.x;   // half as many
+    uint32_t* const hits32 = reinterpret_cast<uint32_t*>(cp_st) + threadIdx.x;   // where nothing is staged
     __shared__ uint32_t colA[9], colP[10], need;
     __shared__ int cmin, cmax;
-    const float h = g.h;
-    const float3 g0 = mk3(g.gx0, g.gy0, g.gz0);
-    const float3 g1 = g0 + mk3((float)g.NX, (float)g.NY, (float)g.NZ) * h;
-    const float3 tmin = g0 + (mk3(h, h, h) + mk3(0.5f * samplespace));
-    const float3 tmax = g1 - (mk3(h, h, h) + mk3(0.5f * samplespace));
     const float re2_skip = re * re * 1.001f;
     const int lane = threadIdx.x & 31;
     // the block's lanes run the same iterations
@@ -335,37 +442,16 @@ __global__ void __launch_bounds__(CP_T, 8) k_correct_springs(Grid g, Cells cl, i
         }
         if (threadIdx.x == 0) { cmin = 0x7fffffff; cmax = -1; need = 0; }
         __syncthreads();
-        float3 ip = xyz(q);
-        int i, j, k; ijkpos(g, ip, i, j, k);
-        // With re below half a cell, a neighbour cell on the far side of the
-        // particle's own half-cell holds only particles whose d2 exceeds
-        // re2_skip (its whole extent is more than 1.002 re away along that
-        // axis, with a margin for the rounding of the cell coordinates), so
-        // every pair in it would be skipped: the cell is not visited.
-        const float3 rel = (ip - g0) / mk3(h, h, h);
-        const float cut_lo = 1.002f * (re / h) + 2e-4f;
-        auto span = [&](float r, int n, int c, int& lo, int& hi) {
-            lo = -1; hi = 1;
-            if (r >= 0 && r < (float)n) {
-                float fr = r - (float)c;
-                if (fr > cut_lo) lo = 0;
-                if (1.0f - fr > cut_lo) hi = 0;
-            }
-        };
-        int ilo, ihi, jlo, jhi, klo, khi;
-        span(rel.x, g.NX, i, ilo, ihi); span(rel.y, g.NY, j, jlo, jhi); span(rel.z, g.NZ, k, klo, khi);
-        // columns outside the grid fall away
-        ilo = max(ilo, -i); ihi = min(ihi, g.NX - 1 - i);
-        jlo = max(jlo, -j); jhi = min(jhi, g.NY - 1 - j);
-        const int k0 = max(k + klo, 0), k1 = min(k + khi, g.NZ - 1);
+        const float3 ip = xyz(q);
+        const CpWindow W(g, ip, re);
         {
             uint32_t cols = 0;
             if (act)
-                for (int di = ilo; di <= ihi; di++)
-                    for (int dj = jlo; dj <= jhi; dj++) cols |= 1u << ((di + 1) * 3 + dj + 1);
+                for (int di = W.ilo; di <= W.ihi; di++)
+                    for (int dj = W.jlo; dj <= W.jhi; dj++) cols |= 1u << ((di + 1) * 3 + dj + 1);
             cols = __reduce_or_sync(0xffffffffu, cols);
-            const int wmin = __reduce_min_sync(0xffffffffu, act ? cid(g, i, j, k0) : 0x7fffffff);
-            const int wmax = __reduce_max_sync(0xffffffffu, act ? cid(g, i, j, k1) : -1);
+            const int wmin = __reduce_min_sync(0xffffffffu, act ? cid(g, W.i, W.j, W.k0) : 0x7fffffff);
+            const int wmax = __reduce_max_sync(0xffffffffu, act ? cid(g, W.i, W.j, W.k1) : -1);
             if (lane == 0 && cols) { atomicMin(&cmin, wmin); atomicMax(&cmax, wmax); atomicOr(&need, cols); }
         }
         __syncthreads();
@@ -386,150 +472,130 @@ __global__ void __launch_bounds__(CP_T, 8) k_correct_springs(Grid g, Cells cl, i
             if (lane == 9) colP[0] = 0;
         }
         __syncthreads();
-        // Two phases keep the warp's lanes together: the scan collects the
-        // pairs within re (a few of the ~64 candidates) in visiting order,
-        // marked where a new cell starts; the spring terms of the collected
-        // pairs are then formed in that order, each cell's sum added to the
-        // total when the next cell starts (a cell without pairs adds +0, a
-        // no-op). A full buffer is drained in the middle of the scan.
-        float3 spring = mk3(0.0f), s = mk3(0.0f);
+        bool direct = false;
+        #pragma unroll
+        for (int c = 0; c < 9; c++) direct |= colP[c + 1] - colP[c] > (uint32_t)CP_CAP;
+        CpSum S;
         int ne = 0;
-        auto pair = [&](float3 o, float m, bool first) {
-            if (first) { spring += s; s = mk3(0.0f); }
-            float3 dd = o - ip;
-            float dist = length(dd);
-            float w = m * smooth_kernel(dist * dist, re);
-            if (dist > 0.1f * re) s += w * (ip - o) / dist;
-        };
-        auto drain16 = [&]() {
+        if (direct) {
+            auto drain = [&]() {
+                for (int e = 0; e < ne; e++) {
+                    const uint32_t x = hits32[e * CP_T], t = x & 0x7fffffffu;
+                    S.pair(ip, xyz(__ldg(pos + t)), __ldg(&vel[t].w), re, x >> 31);
+                }
+                ne = 0;
+            };
+            if (act) {
+                for (int di = W.ilo; di <= W.ihi; di++) for (int dj = W.jlo; dj <= W.jhi; dj++) {
+                    uint32_t bnd[4];
+                    W.bounds(g, cl, di, dj, bnd);
+                    #pragma unroll
+                    for (int u = 0; u < 3; u++) {
+                        uint32_t first = 0x80000000u;
+                        for (uint32_t t = bnd[u]; t < bnd[u + 1]; ++t) {
+                            const float3 dd = xyz(__ldg(pos + t)) - ip;
+                            if (dot(dd, dd) > re2_skip) continue;
+                            hits32[ne * CP_T] = t | first;
+                            first = 0;
+                            if (++ne == CP_BUF) drain();
+                        }
+                    }
+                }
+                drain();
+            }
+        }
+        auto drain = [&]() {
             for (int e = 0; e < ne; e++) {
                 const uint32_t x = hits16[e * CP_T];
                 const uint32_t t = x & 0x7fffu;
-                pair(mk3(sx[t], sy[t], sz[t]), sm[t], x >> 15);
+                S.pair(ip, mk3(sx[t], sy[t], sz[t]), sm[t], re, x >> 15);
             }
             ne = 0;
         };
-        auto drain32 = [&]() {
-            for (int e = 0; e < ne; e++) {
-                const uint32_t x = hits32[e * CP_T], t = x & 0x7fffffffu;
-                pair(xyz(__ldg(pos + t)), __ldg(&vel[t].w), x >> 31);
-            }
-            ne = 0;
-        };
-        for (int c0 = 0, c1; c0 < 9; c0 = c1) {
+        for (int c0 = direct ? 9 : 0, c1; c0 < 9; c0 = c1) {
             const uint32_t P0 = colP[c0];
             c1 = c0;
             while (c1 < 9 && colP[c1 + 1] - P0 <= (uint32_t)CP_CAP) c1++;
-            const bool staged = c1 > c0;
-            if (!staged) c1 = c0 + 1;
-            else {
-                const uint32_t tot = colP[c1] - P0;
-                constexpr int UN = 4;   // loads of a lane in flight together
-                int c = c0;
-                for (uint32_t e0 = threadIdx.x; e0 < tot; e0 += UN * CP_T) {
-                    float4 a[UN]; float m[UN];
-                    #pragma unroll
-                    for (int u = 0; u < UN; u++) {
-                        const uint32_t e = e0 + u * CP_T;
-                        if (e < tot) {
-                            while (e >= colP[c + 1] - P0) c++;
-                            const uint32_t t = colA[c] + (e + P0 - colP[c]);
-                            a[u] = __ldg(pos + t);
-                            m[u] = __ldg(&vel[t].w);
-                        }
+            const uint32_t tot = colP[c1] - P0;
+            constexpr int UN = 4;   // loads of a lane in flight together
+            int c = c0;
+            for (uint32_t e0 = threadIdx.x; e0 < tot; e0 += UN * CP_T) {
+                float4 a[UN]; float m[UN];
+                #pragma unroll
+                for (int u = 0; u < UN; u++) {
+                    const uint32_t e = e0 + u * CP_T;
+                    if (e < tot) {
+                        while (e >= colP[c + 1] - P0) c++;
+                        const uint32_t t = colA[c] + (e + P0 - colP[c]);
+                        a[u] = __ldg(pos + t);
+                        m[u] = __ldg(&vel[t].w);
                     }
-                    #pragma unroll
-                    for (int u = 0; u < UN; u++) {
-                        const uint32_t e = e0 + u * CP_T;
-                        if (e < tot) { sx[e] = a[u].x; sy[e] = a[u].y; sz[e] = a[u].z; sm[e] = m[u]; }
-                    }
+                }
+                #pragma unroll
+                for (int u = 0; u < UN; u++) {
+                    const uint32_t e = e0 + u * CP_T;
+                    if (e < tot) { sx[e] = a[u].x; sy[e] = a[u].y; sz[e] = a[u].z; sm[e] = m[u]; }
                 }
             }
             __syncthreads();
             if (act) {
-                for (int di = ilo; di <= ihi; di++) for (int dj = jlo; dj <= jhi; dj++) {
+                for (int di = W.ilo; di <= W.ihi; di++) for (int dj = W.jlo; dj <= W.jhi; dj++) {
                     const int c = (di + 1) * 3 + dj + 1;
                     if (c < c0 || c >= c1) continue;
-                    // the cells of a (di,dj) column are contiguous
-                    const int cb = cid(g, i + di, j + dj, k0);
                     uint32_t bnd[4];
-                    #pragma unroll
-                    for (int u = 0; u < 4; u++) bnd[u] = __ldg(cl.off + cb + min(u, k1 - k0 + 1));
+                    W.bounds(g, cl, di, dj, bnd);
                     const uint32_t delta = colP[c] - P0 - colA[c];
-                    // beyond re the kernel weight is exactly zero and the pair adds a
-                    // signed zero, which leaves the sum unchanged: skip it (exact test
-                    // with margin: dist*dist >= re*re whenever d2 > 1.001 re*re)
-                    if (staged) {
-                        // eight candidates at a time, two to an instruction, from an even
-                        // slot on; a mask of up to 32 of them, cut to the column's range
-                        // (a contraction of the squares' sum stays far inside the margin)
-                        const float2 nx = make_float2(-ip.x, -ip.x), ny = make_float2(-ip.y, -ip.y), nz = make_float2(-ip.z, -ip.z);
-                        const uint32_t b0 = bnd[0] + delta, b1 = bnd[1] + delta, b2 = bnd[2] + delta, b3 = bnd[3] + delta;
-                        int prev = -1;   // cell of the column's last pair
-                        for (uint32_t t0 = b0 & ~1u; t0 < b3; t0 += 32) {
-                            const uint32_t n = min(b3 - t0, 32u);
-                            uint32_t mask = 0;
-                            for (uint32_t u = 0; u < n; u += 8) {
-                                uint32_t m8 = 0;
-                                #pragma unroll
-                                for (int v = 0; v < 8; v += 2) {
-                                    const uint32_t t = t0 + u + v;
-                                    const float2 dx = add2(*reinterpret_cast<const float2*>(sx + t), nx);
-                                    const float2 dy = add2(*reinterpret_cast<const float2*>(sy + t), ny);
-                                    const float2 dz = add2(*reinterpret_cast<const float2*>(sz + t), nz);
-                                    const float2 d2 = add2(add2(mul2(dx, dx), mul2(dy, dy)), mul2(dz, dz));
-                                    if (!(d2.x > re2_skip)) m8 |= 1u << v;
-                                    if (!(d2.y > re2_skip)) m8 |= 2u << v;
-                                }
-                                mask |= m8 << u;
-                            }
-                            // bits below x of the 32 slots from t0
-                            auto below = [&](uint32_t x) { return x <= t0 ? 0u : x >= t0 + 32 ? 0xffffffffu : (1u << (x - t0)) - 1u; };
-                            mask &= below(b3) & ~below(b0);
-                            if (!mask) continue;
-                            // the first pair of each cell
-                            uint32_t first = 0;
-                            const uint32_t w1 = below(b1), w2 = below(b2);
-                            const uint32_t mq[3] = {mask & w1, mask & w2 & ~w1, mask & ~w2};
+                    // eight candidates at a time, two to an instruction, from an even
+                    // slot on; a mask of up to 32 of them, cut to the column's range
+                    // (a contraction of the squares' sum stays far inside the margin)
+                    const float2 nx = make_float2(-ip.x, -ip.x), ny = make_float2(-ip.y, -ip.y), nz = make_float2(-ip.z, -ip.z);
+                    const uint32_t b0 = bnd[0] + delta, b1 = bnd[1] + delta, b2 = bnd[2] + delta, b3 = bnd[3] + delta;
+                    int prev = -1;   // cell of the column's last pair
+                    for (uint32_t t0 = b0 & ~1u; t0 < b3; t0 += 32) {
+                        const uint32_t n = min(b3 - t0, 32u);
+                        uint32_t mask = 0;
+                        for (uint32_t u = 0; u < n; u += 8) {
+                            uint32_t m8 = 0;
                             #pragma unroll
-                            for (int q = 0; q < 3; q++)
-                                if (mq[q]) {
-                                    if (q != prev) first |= mq[q] & (0u - mq[q]);
-                                    prev = q;
-                                }
-                            while (mask) {
-                                if (ne == CP_BUF) drain16();
-                                const uint32_t bit = mask & (0u - mask);
-                                mask ^= bit;
-                                hits16[ne * CP_T] = (uint16_t)((t0 + (uint32_t)__ffs((int)bit) - 1u) | (first & bit ? 0x8000u : 0u));
-                                ne++;
+                            for (int v = 0; v < 8; v += 2) {
+                                const uint32_t t = t0 + u + v;
+                                const float2 dx = add2(*reinterpret_cast<const float2*>(sx + t), nx);
+                                const float2 dy = add2(*reinterpret_cast<const float2*>(sy + t), ny);
+                                const float2 dz = add2(*reinterpret_cast<const float2*>(sz + t), nz);
+                                const float2 d2 = add2(add2(mul2(dx, dx), mul2(dy, dy)), mul2(dz, dz));
+                                if (!(d2.x > re2_skip)) m8 |= 1u << v;
+                                if (!(d2.y > re2_skip)) m8 |= 2u << v;
                             }
+                            mask |= m8 << u;
                         }
-                    } else {
-                        bool fresh = true;
-                        for (uint32_t t = bnd[0]; t < bnd[3]; ++t) {
-                            const float3 dd = xyz(__ldg(pos + t)) - ip;
-                            fresh |= t == bnd[1] || t == bnd[2];
-                            if (dot(dd, dd) > re2_skip) continue;
-                            hits32[ne * CP_T] = t | (fresh ? 0x80000000u : 0u);
-                            fresh = false;
-                            if (++ne == CP_BUF / 2) drain32();
+                        // bits below x of the 32 slots from t0
+                        auto below = [&](uint32_t x) { return x <= t0 ? 0u : x >= t0 + 32 ? 0xffffffffu : (1u << (x - t0)) - 1u; };
+                        mask &= below(b3) & ~below(b0);
+                        if (!mask) continue;
+                        // the first pair of each cell
+                        uint32_t first = 0;
+                        const uint32_t w1 = below(b1), w2 = below(b2);
+                        const uint32_t mq[3] = {mask & w1, mask & w2 & ~w1, mask & ~w2};
+                        #pragma unroll
+                        for (int q = 0; q < 3; q++)
+                            if (mq[q]) {
+                                if (q != prev) first |= mq[q] & (0u - mq[q]);
+                                prev = q;
+                            }
+                        while (mask) {
+                            if (ne == CP_BUF) drain();
+                            const uint32_t bit = mask & (0u - mask);
+                            mask ^= bit;
+                            hits16[ne * CP_T] = (uint16_t)((t0 + (uint32_t)__ffs((int)bit) - 1u) | (first & bit ? 0x8000u : 0u));
+                            ne++;
                         }
                     }
                 }
-                if (staged) drain16(); else drain32();
+                drain();
             }
             __syncthreads();
         }
-        if (!act) continue;
-        spring += s;
-        spring *= spring_k * re;
-        if (length(dt * spring) > 0.3f * h) ip += h * 0.3f * spring / length(spring);
-        else ip += dt * spring;
-        ip.x = fmaxf(tmin.x, fminf(tmax.x, ip.x));
-        ip.y = fmaxf(tmin.y, fminf(tmax.y, ip.y));
-        ip.z = fmaxf(tmin.z, fminf(tmax.z, ip.z));
-        out[p] = with_xyz(q, ip);
+        if (act) out[p] = with_xyz(q, cp_moved(g, ip, S.spring + S.cell, re, spring_k, samplespace, dt));
     }
 }
 
@@ -980,11 +1046,12 @@ int k_solo_air_update(MpCtx* c) {
 // holds a SOLID particle. The collision reads them only where the solid level
 // set is at most half a cell, and without solid cells it is 3 NX everywhere.
 int k_collide_advect(MpCtx* c, bool skip_empty_solid) {
-    MP_TRY(k_solid_phi(c));   // raises u32_scratch[2] when a cell holds a SOLID particle
+    c->moved = true;
+    MP_TRY(k_solid_phi(c));   // raises u32_scratch[6] when a cell holds a SOLID particle
     bool need_su = true;
     if (skip_empty_solid) {
         uint32_t any = 1;
-        MP_CUDA(c, cudaMemcpyAsync(&any, c->u32_scratch + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+        MP_CUDA(c, cudaMemcpyAsync(&any, c->u32_scratch + 6, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
         MP_CUDA(c, cudaStreamSynchronize(c->stream));
         need_su = any != 0;
     }
@@ -1009,17 +1076,35 @@ int k_correct_pos(MpCtx* c) {
     if (!np) return MP_OK;
     const mp_params& P = c->P;
     KtScope kt(c, MP_KT_CORRECT);
-    MP_CUDA(c, cudaFuncSetAttribute(k_correct_springs, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM));
-    k_correct_springs<<<mp_blocks(np, CP_T), CP_T, CP_SMEM, c->stream>>>(c->G, cells_of(c), np, c->pos, c->vel, c->pos2,
-                                                                     P.correction_radius * c->G.h, P.correction_spring,
-                                                                     P.samplespace, P.dt);
+    const float re = P.correction_radius * c->G.h;
+    // Staging pays where a block's particles share their cells. us, gather and
+    // staged, uniform particles on 64^3 / 128^3:
+    //   4 in a cell that holds any   79  94 /  498  588
+    //   6                           135 131 /  948  951
+    //   8                           198 181 / 1523 1390
+    //   16                          610 532
+    // 256^3 bubble column (8): 19.7 and 18.1 ms. Where a column of three cells is
+    // above CAP nothing is staged, and the gather has all of L1 (1200 a cell: 6.2 and
+    // 7.6 ms). Particles that have moved since the sort spread a block over cells
+    // far apart (melting block, 96^3: 0.6 and 2.0 ms).
+    const double mean = (double)np / std::max(c->sorted_cells, 1u);
+    if (!c->moved && mean >= 6.0 && mean <= CP_CAP / 3) {
+        MP_CUDA(c, cudaFuncSetAttribute(k_correct_springs, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM));
+        k_correct_springs<<<mp_blocks(np, CP_T), CP_T, CP_SMEM, c->stream>>>(c->G, cells_of(c), np, c->pos, c->vel, c->pos2, re,
+                                                                         P.correction_spring, P.samplespace, P.dt);
+    } else {
+        k_correct_gather<<<PB(np)>>>(c->G, cells_of(c), np, c->pos, c->vel, c->pos2, re, P.correction_spring,
+                                     P.samplespace, P.dt);
+    }
     c->launches++;
     MP_CHECK_LAUNCH(c);
     std::swap(c->pos, c->pos2);
+    c->moved = true;
     return MP_OK;
 }
 
 int k_correct_pos_bubble(MpCtx* c) {
+    c->moved = true;
     int sc = c->P.scene;
     int airver = (sc == MP_SCENE_MELTANDBOIL || sc == MP_SCENE_MELTANDBOIL_HIGHRES || sc == MP_SCENE_INTERACTION ||
                   sc == MP_SCENE_ALL) ? 1 : 0;
@@ -1049,6 +1134,7 @@ static int solid_sums(MpCtx* c, int mode, float3 rg0, double out[6]) {
 
 // solidmotion_fixed / solidmotion (spray.cu:2685-2775)
 int k_solid_motion(MpCtx* c) {
+    c->moved = true;
     int np = c->np();
     if (!np) return MP_OK;
     const mp_params& P = c->P;
@@ -1106,6 +1192,7 @@ int k_solid_motion(MpCtx* c) {
 
 // wateradvect (spray.cu:293-305)
 int k_water_advect(MpCtx* c) {
+    c->moved = true;
     int np = c->np();
     if (!np) return MP_OK;
     k_advect_rk2<<<PB(np)>>>(c->G, np, c->pos, c->vel, c->wu[0], c->wu[1], c->wu[2], c->P.dt, c->P.samplespace);
@@ -1245,6 +1332,7 @@ int k_melt(MpCtx* c) {
 }
 
 int k_freeze(MpCtx* c) {
+    c->moved = true;
     int np = c->np();
     MP_CUDA(c, cudaMemsetAsync(c->u32_scratch, 0, sizeof(uint32_t), c->stream));
     if (np) {

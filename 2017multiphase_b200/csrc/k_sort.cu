@@ -46,7 +46,23 @@ __device__ __forceinline__ void load16(const uint32_t* in, size_t n, size_t base
     }
 }
 
-__global__ void __launch_bounds__(SCAN_T) k_scan_reduce(const uint32_t* __restrict__ in, size_t n, uint32_t* __restrict__ part) {
+// the block's entries that are not zero are added to *nonzero
+__device__ __forceinline__ void count_nonzero(const uint32_t (&v)[SCAN_I], uint32_t* nonzero) {
+    int m = 0;
+    #pragma unroll
+    for (int r = 0; r < SCAN_I; r++) m += v[r] != 0;
+    __shared__ uint32_t total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    m = __reduce_add_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&total, (uint32_t)m);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(nonzero, total);
+}
+
+// with `nonzero`, the number of entries that are not zero is added to it
+__global__ void __launch_bounds__(SCAN_T) k_scan_reduce(const uint32_t* __restrict__ in, size_t n, uint32_t* __restrict__ part,
+                                                        uint32_t* __restrict__ nonzero) {
     __shared__ uint32_t ws[SCAN_T / 32];
     size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_I;
     uint32_t v[SCAN_I];
@@ -54,6 +70,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_reduce(const uint32_t* __restri
     uint32_t s = 0;
     #pragma unroll
     for (int r = 0; r < SCAN_I; r++) s += v[r];
+    if (nonzero) count_nonzero(v, nonzero);
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
@@ -93,7 +110,8 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(const uint32_t* __restrict
     }
 }
 
-__global__ void k_scan_single(const uint32_t* __restrict__ in, size_t n, uint32_t* __restrict__ out) {
+__global__ void k_scan_single(const uint32_t* __restrict__ in, size_t n, uint32_t* __restrict__ out,
+                              uint32_t* __restrict__ nonzero) {
     // one block, n <= SCAN_TILE
     __shared__ uint32_t ws[SCAN_T / 32];
     size_t base = (size_t)threadIdx.x * SCAN_I;
@@ -103,6 +121,7 @@ __global__ void k_scan_single(const uint32_t* __restrict__ in, size_t n, uint32_
     uint32_t s = 0;
     #pragma unroll
     for (int r = 0; r < SCAN_I; r++) s += v[r];
+    if (nonzero) count_nonzero(v, nonzero);
     uint32_t inc = warp_incl_scan(s);
     if ((threadIdx.x & 31) == 31) ws[threadIdx.x >> 5] = inc;
     __syncthreads();
@@ -116,9 +135,10 @@ __global__ void k_scan_single(const uint32_t* __restrict__ in, size_t n, uint32_
 }  // namespace
 
 // scan_tmp holds the per-tile partials of every recursion level
-static int scan_rec(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp, size_t tmp_left) {
+static int scan_rec(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp, size_t tmp_left,
+                    uint32_t* nonzero) {
     if (n <= (size_t)SCAN_TILE) {
-        k_scan_single<<<1, SCAN_T, 0, c->stream>>>(in, n, out);
+        k_scan_single<<<1, SCAN_T, 0, c->stream>>>(in, n, out, nonzero);
         c->launches++;
         MP_CHECK_LAUNCH(c);
         return MP_OK;
@@ -127,10 +147,10 @@ static int scan_rec(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n, uint3
     if (2 * nb + 2 > tmp_left) { c->err = "scan: scratch too small"; return MP_ERR_CAPACITY; }
     uint32_t* part = tmp;
     uint32_t* poff = tmp + nb;          // nb + 1 entries
-    k_scan_reduce<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, n, part);
+    k_scan_reduce<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, n, part, nonzero);
     c->launches++;
     MP_CHECK_LAUNCH(c);
-    MP_TRY(scan_rec(c, part, poff, nb, tmp + 2 * nb + 1, tmp_left - (2 * nb + 1)));
+    MP_TRY(scan_rec(c, part, poff, nb, tmp + 2 * nb + 1, tmp_left - (2 * nb + 1), nullptr));
     k_scan_down<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, n, poff, out);
     c->launches++;
     MP_CHECK_LAUNCH(c);
@@ -139,8 +159,8 @@ static int scan_rec(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n, uint3
     return MP_OK;
 }
 
-int mp_scan_u32(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n) {
-    return scan_rec(c, in, out, n, c->scan_tmp, c->scan_tmp_elems);
+int mp_scan_u32(MpCtx* c, const uint32_t* in, uint32_t* out, size_t n, uint32_t* nonzero) {
+    return scan_rec(c, in, out, n, c->scan_tmp, c->scan_tmp_elems, nonzero);
 }
 
 // ---------------------------------------------------------------------------
@@ -299,8 +319,9 @@ static int sort_on_grid(MpCtx* c, float dx, bool grid2x) {
     const int f = grid2x ? 2 : 1, w = f * c->G.NX, hh = f * c->G.NY, d = f * c->G.NZ;
     int np = c->np();
     int ncell = w * hh * d;
-    uint32_t* unsorted = c->u32_scratch + 1;
-    MP_CUDA(c, cudaMemsetAsync(unsorted, 0, sizeof(uint32_t), c->stream));
+    uint32_t *unsorted = c->u32_scratch + 1, *in_use = unsorted + 1;
+    MP_CUDA(c, cudaMemsetAsync(unsorted, 0, 2 * sizeof(uint32_t), c->stream));
+    c->moved = false;
     c->types_stale = false;
     c->sorted_np = np;
     c->sorted_2x = grid2x;
@@ -310,10 +331,12 @@ static int sort_on_grid(MpCtx* c, float dx, bool grid2x) {
         c->launches++;
         MP_CHECK_LAUNCH(c);
     }
-    MP_TRY(mp_scan_u32(c, c->cell_cnt, c->cell_off, (size_t)ncell));
-    uint32_t h_unsorted = 1;
-    MP_CUDA(c, cudaMemcpyAsync(&h_unsorted, unsorted, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+    MP_TRY(mp_scan_u32(c, c->cell_cnt, c->cell_off, (size_t)ncell, grid2x ? nullptr : in_use));
+    uint32_t h[2] = {1, 0};
+    MP_CUDA(c, cudaMemcpyAsync(h, unsorted, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     MP_CUDA(c, cudaStreamSynchronize(c->stream));
+    const uint32_t h_unsorted = h[0];
+    if (!grid2x) c->sorted_cells = h[1];
     c->work[h_unsorted ? MP_WC_SORT_FULL : MP_WC_SORT_FAST]++;
     if (!h_unsorted) {
         // already in cell order: the stable sort is the identity permutation;
