@@ -131,10 +131,9 @@ static int create_impl(MpCtx* c, const mp_params* p) {
     MP_CUDA(c, cudaMemset(c->cell_cnt, 0, sizeof(uint32_t) * (n8 + 1)));
     MP_CUDA(c, cudaMemset(c->cell_off, 0, sizeof(uint32_t) * (n8 + 1)));
     {
-        const size_t bricks = (size_t)((p->nx + 3) / 4) * ((p->ny + 3) / 4) * ((p->nz + 3) / 4);
-        c->air_brick_words = (bricks + 31) / 32;
-        MP_TRY(dalloc_t(c, &c->air_brick, c->air_brick_words));
-        MP_CUDA(c, cudaMemset(c->air_brick, 0, sizeof(uint32_t) * c->air_brick_words));
+        c->air_bricks = (size_t)((p->nx + 3) / 4) * ((p->ny + 3) / 4) * ((p->nz + 3) / 4);
+        MP_TRY(dalloc_t(c, &c->air_brick, c->air_bricks));
+        MP_CUDA(c, cudaMemset(c->air_brick, 0, c->air_bricks));
         c->cell_bits_half = (n + 31) / 32 + 2;
         MP_TRY(dalloc_t(c, &c->cell_bits, 2 * c->cell_bits_half));
         MP_CUDA(c, cudaMemset(c->cell_bits, 0, sizeof(uint32_t) * 2 * c->cell_bits_half));

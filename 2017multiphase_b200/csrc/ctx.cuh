@@ -89,8 +89,8 @@ struct MpCtx {
     uint32_t *keys = 0, *perm = 0;
     uint32_t *cell_cnt = 0, *cell_off = 0;   // sized for the 2x marching-cubes grid
     uint8_t *tmask = 0;
-    uint32_t *air_brick = 0;     // bit per brick (4^3 cells, 8^3 of the 2x grid) holding an AIR/AIRSOLO particle (last sort)
-    size_t air_brick_words = 0;
+    uint8_t *air_brick = 0;      // 1 for each brick (4^3 cells, 8^3 of the 2x grid) holding an AIR/AIRSOLO particle (last sort)
+    size_t air_bricks = 0;
     // a bit per cell of the simulation grid (last sort), a spare word before and
     // after: AIR/AIRSOLO, then FLUID/SOLID cell_bits_half words further
     uint32_t *cell_bits = 0;

@@ -80,7 +80,7 @@ __device__ __forceinline__ float nearest2(const Grid& g, const uint32_t* __restr
 // 256^3 3.5 -> 2.2 ms, 32^3 135 -> 82 us.
 __global__ void __launch_bounds__(256) k_genlevelset(Grid g, const uint32_t* __restrict__ off, const float4* __restrict__ pos,
                                                      float* __restrict__ lsf, float* __restrict__ lsa,
-                                                     int8_t* __restrict__ mark, const uint32_t* __restrict__ air_brick,
+                                                     int8_t* __restrict__ mark, const uint8_t* __restrict__ air_brick,
                                                      const uint32_t* __restrict__ bits, size_t half_words) {
     const float h = g.h, r = 0.5f * h;
     const int stride = (int)(gridDim.x * blockDim.x), t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -105,8 +105,7 @@ __global__ void __launch_bounds__(256) k_genlevelset(Grid g, const uint32_t* __r
             for (int bi = bi0; bi <= bi1; bi++)
                 for (int bj = bj0; bj <= bj1; bj++)
                     for (int bk = bk0; bk <= bk1; bk++) {
-                        const int br = (bi * bh + bj) * bw + bk;
-                        near |= (__ldg(air_brick + (br >> 5)) >> (br & 31)) & 1u;
+                        near |= __ldg(air_brick + (bi * bh + bj) * bw + bk) != 0;
                     }
             if (near) m2 = nearest2(g, off, pos, bits, MP_TYPEAIR, MP_TYPEAIRSOLO, i, j, k, gp);
         }

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256, 6) k_mc_density_solid(McGrid m, Tiles T, 
 template <int SURF, bool GAS2, bool INRANGE>
 __global__ void __launch_bounds__(256, 4) k_mc_pairs(McGrid m, Tiles T, Cells cl, const float4* __restrict__ pos,
                                                      float* __restrict__ dens, int scene, float* __restrict__ dens2,
-                                                     const uint32_t* __restrict__ air_brick) {
+                                                     const uint8_t* __restrict__ air_brick) {
     const float hm = m.hm, R = hm * 2, RR = R * R;
     const float tiny = RR * 8.7e-19f;   // below it dis^2 does not change R^2 - dis^2
     const uint32_t gas_types = (1u << MP_TYPEAIR) | (scene != MP_SCENE_INTERACTION ? (1u << MP_TYPEAIRSOLO) : 0u);
@@ -125,8 +125,7 @@ __global__ void __launch_bounds__(256, 4) k_mc_pairs(McGrid m, Tiles T, Cells cl
             for (int a = i0; a <= i1; a++)
                 for (int b = b0; b <= b1; b++)
                     for (int c = k0; c <= k1; c++) {
-                        const int br = (a * bh + b) * bw + c;
-                        air |= (__ldg(air_brick + (br >> 5)) >> (br & 31)) & 1u;
+                        air |= __ldg(air_brick + (a * bh + b) * bw + c) != 0;
                     }
         }
         const bool warp_air = __any_sync(0xffffffffu, air);

@@ -39,7 +39,7 @@ constexpr int P2G_CAP = 320, P2G_AIR_CAP = 192;
 // in the same order with the same arithmetic as the one-thread-per-face-triple
 // gather, so the fields are bit-identical.
 // Air is sparse: a warp whose windows touch no 4x4x4-cell brick with an air
-// particle (the bit map of the last sort) writes 0, a column without an air
+// particle (marked by the last sort) writes 0, a column without an air
 // cell is skipped, and only the air particles of a chunk are staged (its places
 // by a running count, so a lane's part of the chunk is again a range).
 // 256^3: water 17.6 -> 10.9 ms, air 2.6 -> 2.4 ms; 32^3: water 87 -> 51 us, air 222 -> 110 us.
@@ -47,7 +47,7 @@ template <bool AIR, int CAP>
 __global__ void __launch_bounds__(256, AIR ? 3 : 2) k_p2g_staged(Grid g, Cells cl, const float4* __restrict__ pos,
                                                                const float4* __restrict__ vel, float* __restrict__ ux,
                                                                float* __restrict__ uy, float* __restrict__ uz,
-                                                               const uint32_t* __restrict__ air_brick) {
+                                                               const uint8_t* __restrict__ air_brick) {
     constexpr int R = AIR ? 2 : 1;     // union window -R..R
     constexpr int HI = AIR ? 1 : 0;    // upper bound along the face normal
     extern __shared__ float4 p2g_sm[];
@@ -78,8 +78,7 @@ __global__ void __launch_bounds__(256, AIR ? 3 : 2) k_p2g_staged(Grid g, Cells c
                 for (int bi = bi0; bi <= bi1; bi++)
                     for (int bj = bj0; bj <= bj1; bj++)
                         for (int bk = bk0; bk <= bk1; bk++) {
-                            const int br = (bi * bh + bj) * bw + bk;
-                            near |= (__ldg(air_brick + (br >> 5)) >> (br & 31)) & 1u;
+                            near |= __ldg(air_brick + (bi * bh + bj) * bw + bk) != 0;
                         }
             }
         }
