@@ -279,6 +279,7 @@ extern "C" int mp_set_stream(void* ctx, void* stream) {
     MP_CUDA(c, cudaStreamSynchronize(c->stream));
     if (c->own_stream) { cudaStreamDestroy(c->stream); c->own_stream = false; }
     c->stream = (cudaStream_t)stream;
+    c->cg_res_off = false;
     return MP_OK;
 }
 extern "C" int mp_get_stream(void* ctx, void** stream) {
@@ -699,6 +700,11 @@ void kt_end(MpCtx* c, int cls, cudaEvent_t ev_end) {
     if (!ev_end) return;
     cudaEventRecord(ev_end, c->stream);
     if (c->kt_pending[cls].size() > 4096) { cudaStreamSynchronize(c->stream); kt_harvest(c, cls); }
+}
+void kt_cancel(MpCtx* c, int cls, cudaEvent_t ev_end) {
+    if (!ev_end) return;
+    c->kt_pool.push_back(c->kt_pending[cls].back());
+    c->kt_pending[cls].pop_back();
 }
 extern "C" int mp_kernel_timing(void* ctx, int cls, int enable) {
     MpCtx* c = C(ctx); CTX_OR_ARG(c);

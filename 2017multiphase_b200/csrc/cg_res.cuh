@@ -44,7 +44,8 @@
 // the FP64 dot products add their terms in another order.
 //
 // The launch is cooperative (its CTAs wait on one another) and every wait is
-// bounded: after RES_WAIT_NS the CTA raises DONE_TIMEOUT and returns.
+// bounded: after RES_WAIT_NS the CTA raises DONE_TIMEOUT and returns, and the
+// solve is done again by the passes.
 #pragma once
 
 namespace {
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(RES_T, 1)
     using Grp = ResGroup<R>;
     constexpr int V = Grp::V;
     const Grid& g = op.g;
-    const int NZ = g.NZ, KG = G.KG, RS = KG * V, nblk = gridDim.x;
+    const int NZ = g.NZ, KG = G.KG, nblk = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int bi = blockIdx.x / G.nbj, bj = blockIdx.x - bi * G.nbj;
     const int i0 = bi * G.ti, j0 = bj * G.tj;

@@ -74,6 +74,8 @@ struct MpCtx {
     uint64_t* cg_exch = 0;            // its halo rows and partial sums
     size_t cg_exch_words = 0;
     uint32_t cg_epoch = 1;            // first tag that no exchange has used
+    bool cg_res_off = false;          // an exchange ran out of time on this stream
+    int cg_res_missing = 0;           // blocks left out of its launch (tests of its waits)
     int cg_tma_chunk = 0;
     float *gfm_beta = 0;         // ghost-fluid face weights (x, y, z faces), allocated on first use
     float *gfm_s = 0;            // its Jacobi scaling per cell
@@ -189,6 +191,7 @@ struct NvtxRange {
 // kernel-class timing (events around launches on the context stream)
 void kt_begin(MpCtx* c, int cls, cudaEvent_t* ev_end);
 void kt_end(MpCtx* c, int cls, cudaEvent_t ev_end);
+void kt_cancel(MpCtx* c, int cls, cudaEvent_t ev_end);   // the launch since kt_begin did not happen
 struct KtScope {
     MpCtx* c; int cls; cudaEvent_t e1 = 0;
     KtScope(MpCtx* c_, int cls_) : c(c_), cls(cls_) { kt_begin(c, cls, &e1); }
@@ -235,7 +238,7 @@ int k_melt(MpCtx* c);
 int k_freeze(MpCtx* c);
 int k_mc(MpCtx* c, int surface, bool keep_field = true);
 int k_mc_fluid_gas(MpCtx* c);
-int k_cg_res_setup(MpCtx* c);
+int k_cg_res_setup(MpCtx* c, int sms = 0);
 int k_cg_solve(MpCtx* c, const int8_t* mark, float* x, const float* b, int maxiter, int tolmode, float tol, int* iters,
                double* res);
 int k_cg_solve(MpCtx* c, const int8_t* mark, double* x, const double* b, int maxiter, int tolmode, float tol,

@@ -896,18 +896,23 @@ static Red red_of(MpCtx* c) {
     return Red{c->red, c->red_count, c->scal, reinterpret_cast<unsigned int*>(c->red_count + 1)};
 }
 
-// The on-chip solve's plans and exchange buffer (cg_res.cuh), made once: the
-// grid of a context is fixed.
-int k_cg_res_setup(MpCtx* c) {
-    int sms = 0, smem = 0, coop = 0;
-    MP_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+// The on-chip solve's plans for FP32 and FP64 vectors on so many SMs with so much
+// shared memory a block
+static void cg_res_plans(const Grid& g, int sms, size_t smem, ResPlan* p32, ResPlan* p64) {
+    const size_t room = smem - 1024;   // the kernel's static shared memory
+    *p32 = res_plan<float>(g, sms, room, true);
+    if (!p32->nblk || p32->Q > RES_ONE_Q) *p32 = res_plan<float>(g, sms, room, false);
+    *p64 = res_plan<double>(g, sms, room, false);
+}
+// The plans and the exchange buffer (cg_res.cuh), made once: the grid of a
+// context is fixed. sms: 0, or another number of SMs than the device's.
+int k_cg_res_setup(MpCtx* c, int sms) {
+    int smem = 0, coop = 0;
+    if (!sms) MP_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
     MP_CUDA(c, cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     MP_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
     if (!coop || !c->cg_use_res) return MP_OK;
-    const size_t room = (size_t)smem - 1024;   // the kernel's static shared memory
-    c->res_plan32 = res_plan<float>(c->G, sms, room, true);
-    if (!c->res_plan32.nblk || c->res_plan32.Q > RES_ONE_Q) c->res_plan32 = res_plan<float>(c->G, sms, room, false);
-    c->res_plan64 = res_plan<double>(c->G, sms, room, false);
+    cg_res_plans(c->G, sms, (size_t)smem, &c->res_plan32, &c->res_plan64);
     const size_t words = std::max(c->res_plan32.nblk ? res_exch_words(c->res_plan32) : 0,
                                   c->res_plan64.nblk ? res_exch_words(c->res_plan64) : 0);
     if (!words) return MP_OK;
@@ -916,13 +921,41 @@ int k_cg_res_setup(MpCtx* c) {
     MP_CUDA(c, cudaMemset(c->cg_exch, 0, sizeof(uint64_t) * c->cg_exch_words));
     return MP_OK;
 }
+// For tests, on the host: what a grid's solve is planned as on so many SMs of
+// 227 KB: blocks, groups a thread (as built), one exchange an iteration, tile.
+extern "C" int mp_internal_cg_plan(int nx, int ny, int nz, int sms, int fp64, int32_t* out) {
+    Grid g{};
+    g.NX = nx; g.NY = ny; g.NZ = nz;
+    ResPlan p32, p64;
+    cg_res_plans(g, sms, 232448, &p32, &p64);
+    const ResPlan& P = fp64 ? p64 : p32;
+    out[0] = P.nblk; out[1] = P.Q; out[2] = P.one; out[3] = P.g.ti; out[4] = P.g.tj;
+    return MP_OK;
+}
+// For tests: plans for another number of SMs (0: the device's), the first tag,
+// and how many of a plan's blocks are left out of the launch.
+extern "C" int mp_internal_cg_setup(void* ctx, int sms, uint32_t epoch, int missing) {
+    MpCtx* c = static_cast<MpCtx*>(ctx);
+    MP_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (c->cg_exch) cudaFree(c->cg_exch);
+    c->cg_exch = nullptr;
+    MP_TRY(k_cg_res_setup(c, sms));
+    c->cg_epoch = epoch;
+    c->cg_res_missing = missing;
+    c->cg_res_off = false;
+    return MP_OK;
+}
 
-// The solve in one launch, when the grid fits on chip; *taken tells.
+// The solve in one launch, when the grid fits on chip; *taken tells. It is not
+// taken either when the launch is refused (its blocks have to be resident together,
+// and a stream may be limited to part of the SMs) or when an exchange runs out of
+// time: the passes need neither. After the second the context stays with the
+// passes, as the next solve would wait as long, until it is given another stream.
 template <class R, class Op>
 static int run_cg_res(MpCtx* c, const Op& op, R* x, const R* b, int maxiter, int tolmode, float tol, int* iters_out,
                       double* res_out, int kt_class, bool* taken) {
     const ResPlan& P = sizeof(R) == 4 ? c->res_plan32 : c->res_plan64;
-    *taken = P.nblk > 0 && maxiter < (1 << 28);
+    *taken = P.nblk > 0 && !c->cg_res_off && maxiter < (1 << 28);
     if (!*taken) return MP_OK;
     void (*kern)(Op, ResGeom, const R*, R*, uint64_t*, uint64_t*, Red, int, float, int, uint32_t) = nullptr;
     if constexpr (sizeof(R) == 4) {
@@ -960,11 +993,16 @@ static int run_cg_res(MpCtx* c, const Op& op, R* x, const R* b, int maxiter, int
     uint64_t *slots = c->cg_exch, *exch = c->cg_exch + RES_SLOT_WORDS;
     uint32_t epoch = c->cg_epoch;
     void* args[] = {&o, &g, &b, &x, &exch, &slots, &Rd, &tolmode, &tol, &maxiter, &epoch};
-    {
-        KtScope kt(c, kt_class);
-        MP_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(P.nblk), dim3(RES_T), args,
-                                               P.smem, s));
+    cudaEvent_t timed = 0;
+    kt_begin(c, kt_class, &timed);
+    if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(P.nblk - c->cg_res_missing), dim3(RES_T), args,
+                                    P.smem, s) != cudaSuccess) {
+        cudaGetLastError();   // an error that stays comes back from the passes
+        kt_cancel(c, kt_class, timed);
+        *taken = false;
+        return MP_OK;
     }
+    kt_end(c, kt_class, timed);
     c->launches++;
     unsigned int hflag[F_COUNT] = {0, 0};
     double rr = 0;
@@ -974,8 +1012,9 @@ static int run_cg_res(MpCtx* c, const Op& op, R* x, const R* b, int maxiter, int
     if (hflag[F_DONE] == DONE_TIMEOUT || hflag[F_DONE] == 0xffffffffu) {
         MP_CUDA(c, cudaMemsetAsync(c->cg_exch, 0, sizeof(uint64_t) * c->cg_exch_words, s));
         c->cg_epoch = 1;
-        c->err = "cg: an exchange between thread blocks ran out of time";
-        return MP_ERR_TIMEOUT;
+        c->cg_res_off = true;
+        *taken = false;
+        return MP_OK;
     }
     c->cg_epoch += 2u * hflag[F_ITERS] + 8u;
     *iters_out = (int)hflag[F_ITERS];
