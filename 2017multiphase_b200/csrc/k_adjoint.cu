@@ -1243,7 +1243,7 @@ int ad_g2p_adj(MpCtx* c, const Grid& g, const uint32_t* off, const T* xs4, const
     return MP_OK;
 }
 // the splat kernel's two quotients, 1.96 / r2 and that over r2 again, for r2 in
-// [1e-4, 1.96]: both equal / on every float of that range
+// [1e-4, 1.96]
 __device__ __forceinline__ float ad_quot(float a, float r2) { return quot_in_range(a, r2); }
 __device__ __forceinline__ double ad_quot(double a, double r2) { return a / r2; }
 // per face ub/W of a splat (0 where the face took no weight): the factor every

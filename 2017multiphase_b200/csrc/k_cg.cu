@@ -82,25 +82,6 @@ __device__ __forceinline__ bool finish_sum(const Red& R, double mine, double* to
 __device__ __forceinline__ bool inner(const Grid& g, int i, int j, int k) {
     return i > 0 && i < g.NX - 1 && j > 0 && j < g.NY - 1 && k > 0 && k < g.NZ - 1;
 }
-// s / h^2 by the reciprocal: with c = 1/h^2 rounded to nearest, q = s c and its
-// exact remainder s - q h^2 (one fused operation), q + c times the remainder is
-// the correctly rounded quotient (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990). The remainder is
-// exact for |s| above 4e-31 (FP32); below, the last bit may differ. Three
-// operations, where a division by a variable takes about 5 cycles of an SM per
-// warp and in FP64 a call (around which registers spilled).
-struct CgQuot {
-    float f = 0.0f, hf = 0.0f;    // 1/h^2 (0: h^2 too far from one, divide) and h^2
-    double d = 0.0, hd = 0.0;
-};
-__device__ __forceinline__ float cg_quot(float s, const CgQuot& c) {
-    const float q = s * c.f;
-    return fabsf(q) <= 3.4e38f ? __fmaf_rn(__fmaf_rn(-q, c.hf, s), c.f, q) : q;
-}
-__device__ __forceinline__ double cg_quot(double s, const CgQuot& c) {
-    const double q = s * c.d;
-    return fabs(q) <= 1.7e308 ? __fma_rn(__fma_rn(-q, c.hd, s), c.d, q) : q;
-}
 // computeAx_bubble (spray_k.cu:3423-3447): rows over FLUID and AIR cells;
 // with air = false, computeAx (spray_k.cu:2300-2322) of the single-phase
 // solve: rows over FLUID cells only, AIR cells a zero-pressure region

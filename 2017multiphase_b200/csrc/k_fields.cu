@@ -120,12 +120,6 @@ __device__ __forceinline__ void solvedistance(float a, float b, float c, float& 
         d = (a + b + c + sqrtf(3 - (a - b) * (a - b) - (a - c) * (a - c) - (b - c) * (b - c))) / 3;
     if (d < x) x = d;
 }
-// x / 3, correctly rounded: the reciprocal's estimate and its exact remainder
-// (see quot_in_range); equal to / on every float from 2^-100 to 2^100
-__device__ __forceinline__ float third(float x) {
-    const float r = 1.0f / 3.0f, q = x * r;
-    return __fmaf_rn(__fmaf_rn(-3.0f, q, x), r, q);
-}
 // A cell whose six neighbours are all at least its value and settled keeps it:
 // an octant with m = min(a,b,c) >= res cannot lower res when its result is
 // provably not below res: the result is m + 1 rounded (>= m) when that is not above the maximum; otherwise
