@@ -36,13 +36,13 @@ def names_kt(mp):
             mp.KT_CORRECT: "k_correct_springs"}
 
 
-# DRAM bytes per launch from ncu captures (dram__bytes_read.sum + dram__bytes_write.sum),
-# as functions of (cells, particles): the capture's bytes scaled by the units a
-# launch processes
+# DRAM bytes per launch from ncu captures (dram__bytes_read.sum + dram__bytes_write.sum)
+# and the grid that they were captured at; other grids have none (what L2 saves
+# does not grow with the grid)
 TRAFFIC_PER_LAUNCH = {
-    # the TMA CG passes captured at 224^3 (--profile-case cg): 120.6 MB and 174.1 MB per launch
-    "k_cg_dir": lambda n, np_: 120.59e6 * n / 224 ** 3,
-    "k_cg_upd": lambda n, np_: 174.06e6 * n / 224 ** 3,
+    # the TMA CG passes on the liquid slab of --profile-case cg --n 256
+    "k_cg_dir": (256 ** 3, 187.6e6),
+    "k_cg_upd": (256 ** 3, 281.0e6),
 }
 
 
@@ -583,28 +583,40 @@ def main():
              # read each position record and neighbour mass, write the corrected record; cell ranges
              mp.KT_CORRECT: ("k_correct_springs (particle spacing spring)", (36 * npart + 4 * n) * kt[mp.KT_CORRECT][1],
                              kt[mp.KT_CORRECT][1])}
+    # a grid that fits on chip has its whole solve, all iterations of it, in one
+    # launch of the first class, whose vectors do not go through HBM
+    on_chip = kt[mp.KT_CG_STENCIL][1] > 0 and kt[mp.KT_CG_UPDATE][1] == 0
+    if on_chip:
+        model[mp.KT_CG_STENCIL] = ("k_cg_res (a whole pressure solve on chip)", None, kt[mp.KT_CG_STENCIL][1])
     dom = max(model, key=lambda k: kt[k][0])
     ms_k = kt[dom][0]
     units = max(model[dom][2], 1)
     per_unit_s = ms_k / 1e3 / units
-    alg = model[dom][1] / units
-    achieved = alg / per_unit_s / 1e9
-    traffic = TRAFFIC_PER_LAUNCH.get(names_kt(mp)[dom])
-    cg_ms = kt[mp.KT_CG_STENCIL][0] + kt[mp.KT_CG_UPDATE][0]
-    pcg_gbs = (CG_DIR_BYTES_PER_CELL + CG_UPD_BYTES_PER_CELL) * n * max(wc["cg_iters"], 1) / (cg_ms / 1e3) / 1e9
     names = names_kt(mp)
+    if on_chip:
+        names[mp.KT_CG_STENCIL] = "k_cg_res"
+    alg = model[dom][1] / units if model[dom][1] is not None else None
+    achieved = alg / per_unit_s / 1e9 if alg is not None else None
+    cells_captured, traffic = TRAFFIC_PER_LAUNCH.get(names[dom], (0, None))
+    if cells_captured != n:
+        traffic = None
+    cg_ms = kt[mp.KT_CG_STENCIL][0] + kt[mp.KT_CG_UPDATE][0]
+    pcg_gbs = None
+    if not on_chip:
+        pcg_gbs = (CG_DIR_BYTES_PER_CELL + CG_UPD_BYTES_PER_CELL) * n * max(wc["cg_iters"], 1) / (cg_ms / 1e3) / 1e9
     psrc = f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback"
-    roof = {"kernel": model[dom][0], "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "peak_source": psrc,
-            "traffic": (traffic(n, npart) if traffic else None), "algorithmic_bytes_per_launch": alg,
-            "avg_launch_ms": per_unit_s * 1e3}
+    roof = {"kernel": model[dom][0], "bound": "hbm" if alg is not None else "latency", "achieved": achieved, "peak": peak,
+            "unit": "GB/s", "frac": achieved / peak if alg is not None else None, "peak_source": psrc,
+            "traffic": traffic, "algorithmic_bytes_per_launch": alg, "avg_launch_ms": per_unit_s * 1e3}
     cls_table = {}
     for k, (nm, b, u) in model.items():
         ms_c, nl_c = kt[k]
         if nl_c and ms_c > 0:
-            a = b / (ms_c / 1e3) / 1e9
+            a = b / (ms_c / 1e3) / 1e9 if b is not None else None
             cls_table[names[k]] = {"ms": ms_c, "launches": nl_c, "work_units": u, "algorithmic_GBps": a,
-                                   "frac": a / peak}
+                                   "frac": a / peak if b is not None else None}
+    if on_chip:
+        cls_table["k_cg_res"]["us_per_iteration"] = 1e3 * kt[mp.KT_CG_STENCIL][0] / max(wc["cg_iters"], 1)
     cls_table["sort"]["calls_reordering"] = wc["sort_full"]
     cls_table["sort"]["calls_in_order"] = wc["sort_fast"]
     cls_table["steps"] = class_steps
@@ -617,8 +629,9 @@ def main():
            "scaling": "weak", "vs_baseline": None, "dtype": "f32 (CG dots, alpha/beta in f64)", "data": "synthetic",
            "config": workload_config(p, npart0, args.seed, world),
            "roofline": roof, "pcg_hbm_gbs": pcg_gbs,
-           "pcg_roofline": {"achieved": pcg_gbs, "peak": peak, "unit": "GB/s", "frac": pcg_gbs / peak,
-                            "note": "both CG passes, 34 B/cell/iteration algorithmic, per CG iteration"},
+           "pcg_roofline": None if on_chip else
+           {"achieved": pcg_gbs, "peak": peak, "unit": "GB/s", "frac": pcg_gbs / peak,
+            "note": "both CG passes, 34 B/cell/iteration algorithmic, per CG iteration"},
            "cg_iters_per_step": cg_iters / max(args.steps, 1),
            "mesh": {"verts": [int(v) for v in st.mc_verts], "triangles": [int(v) // 3 for v in st.mc_indices]},
            "kernel_classes": cls_table,
