@@ -210,9 +210,12 @@ typedef struct mp_state {
 #define MP_MC_FLUID 1
 #define MP_MC_GAS   2
 
-/* Kernel classes whose launches can be timed with CUDA events. */
-#define MP_KT_CG_STENCIL   0   /* pressure CG: A p and p.Ap                */
-#define MP_KT_CG_UPDATE    1   /* pressure CG: x, r update and r.r          */
+/* Kernel classes whose launches can be timed with CUDA events. A CG solve
+ * (pressure or heat) is a launch of each of the first two classes per iteration,
+ * or, on a grid whose vectors fit on chip, one launch of MP_KT_CG_STENCIL for
+ * the whole solve and none of MP_KT_CG_UPDATE. */
+#define MP_KT_CG_STENCIL   0   /* CG: A p and p.Ap; or the whole solve      */
+#define MP_KT_CG_UPDATE    1   /* CG: x, r update and r.r                   */
 #define MP_KT_P2G          2   /* water + air particle-to-grid gather       */
 #define MP_KT_G2P          3   /* FLIP grid-to-particle                     */
 #define MP_KT_SORT         4   /* hash + counting sort + reorder            */
