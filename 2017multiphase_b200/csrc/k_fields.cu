@@ -97,16 +97,9 @@ __global__ void __launch_bounds__(256) k_genlevelset(Grid g, const uint32_t* __r
         } else {
             // no brick that the window (i-2..i+2, ...) touches holds an air
             // particle: the air distance stays at its cap
-            bool near = false;
-            const int bw = (g.NZ + 3) / 4, bh = (g.NY + 3) / 4;
-            const int bi0 = max(i - 2, 0) >> 2, bi1 = min(i + 2, g.NX - 1) >> 2;
-            const int bj0 = max(j - 2, 0) >> 2, bj1 = min(j + 2, g.NY - 1) >> 2;
-            const int bk0 = max(k - 2, 0) >> 2, bk1 = min(k + 2, g.NZ - 1) >> 2;
-            for (int bi = bi0; bi <= bi1; bi++)
-                for (int bj = bj0; bj <= bj1; bj++)
-                    for (int bk = bk0; bk <= bk1; bk++) {
-                        near |= __ldg(air_brick + (bi * bh + bj) * bw + bk) != 0;
-                    }
+            const bool near = brick_marked(air_brick, (g.NY + 3) / 4, (g.NZ + 3) / 4, max(i - 2, 0) >> 2,
+                                           min(i + 2, g.NX - 1) >> 2, max(j - 2, 0) >> 2, min(j + 2, g.NY - 1) >> 2,
+                                           max(k - 2, 0) >> 2, min(k + 2, g.NZ - 1) >> 2);
             if (near) m2 = nearest2(g, off, pos, bits, MP_TYPEAIR, MP_TYPEAIRSOLO, i, j, k, gp);
         }
         const float d = sqrtf(m2), far = 2.5f * h;

@@ -116,18 +116,9 @@ __global__ void __launch_bounds__(256, 4) k_mc_pairs(McGrid m, Tiles T, Cells cl
         if (!__any_sync(0xffffffffu, live)) continue;
         const int j0 = 1 + 2 * jt;
         i += 1; k += 1;   // the nodes inside the border
-        bool air = false;
-        if (live) {
-            const int bw = (m.NZMC + 7) / 8, bh = (m.NYMC + 7) / 8;
-            const int i0 = max(i - 2, 0) >> 3, i1 = min(i + 1, m.NXMC - 1) >> 3;
-            const int b0 = max(j0 - 2, 0) >> 3, b1 = min(j0 + 2, m.NYMC - 1) >> 3;
-            const int k0 = max(k - 2, 0) >> 3, k1 = min(k + 1, m.NZMC - 1) >> 3;
-            for (int a = i0; a <= i1; a++)
-                for (int b = b0; b <= b1; b++)
-                    for (int c = k0; c <= k1; c++) {
-                        air |= __ldg(air_brick + (a * bh + b) * bw + c) != 0;
-                    }
-        }
+        const bool air = live && brick_marked(air_brick, (m.NYMC + 7) / 8, (m.NZMC + 7) / 8, max(i - 2, 0) >> 3,
+                                              min(i + 1, m.NXMC - 1) >> 3, max(j0 - 2, 0) >> 3, min(j0 + 2, m.NYMC - 1) >> 3,
+                                              max(k - 2, 0) >> 3, min(k + 1, m.NZMC - 1) >> 3);
         const bool warp_air = __any_sync(0xffffffffu, air);
         const float px = (float)i * hm, py0 = (float)j0 * hm, py1 = (float)(j0 + 1) * hm, pz = (float)k * hm;
         // the cells k-2 .. k+1 inside the grid, as bounds of the off entries

@@ -69,18 +69,9 @@ __global__ void __launch_bounds__(256, AIR ? 3 : 2) k_p2g_staged(Grid g, Cells c
         FaceSums F;
         bool near = true;
         if (AIR) {
-            near = false;
-            if (act) {
-                const int bw = (g.NZ + 3) / 4, bh = (g.NY + 3) / 4;
-                const int bi0 = max(i - R, 0) >> 2, bi1 = min(i + R, g.NX - 1) >> 2;
-                const int bj0 = max(j - R, 0) >> 2, bj1 = min(j + R, g.NY - 1) >> 2;
-                const int bk0 = max(k - R, 0) >> 2, bk1 = min(k + R, g.NZ - 1) >> 2;
-                for (int bi = bi0; bi <= bi1; bi++)
-                    for (int bj = bj0; bj <= bj1; bj++)
-                        for (int bk = bk0; bk <= bk1; bk++) {
-                            near |= __ldg(air_brick + (bi * bh + bj) * bw + bk) != 0;
-                        }
-            }
+            near = act && brick_marked(air_brick, (g.NY + 3) / 4, (g.NZ + 3) / 4, max(i - R, 0) >> 2, min(i + R, g.NX - 1) >> 2,
+                                       max(j - R, 0) >> 2, min(j + R, g.NY - 1) >> 2, max(k - R, 0) >> 2,
+                                       min(k + R, g.NZ - 1) >> 2);
         }
         if (__any_sync(0xffffffffu, near)) {
             const float3 gpx = mk3((float)i, (float)j + 0.5f, (float)k + 0.5f);
