@@ -16,9 +16,11 @@
 // the new r (about 1e-7 / sqrt(cells) of r . r). The true r . r comes with the next
 // exchange. Where its beta rounds to another float, in a few of a hundred iterations,
 // p and z are formed again from the last p, which is kept beside the new one;
-// alpha, the stop rule and the count use the true r . r too, so the vectors are
-// those of two exchanges bit for bit. (Left alone, one float of beta off changes
-// where the iteration stops: 2.5e-4 in a velocity at a tolerance of 1e-6.)
+// alpha, the stop rule and the count use the true r . r too. So nothing is
+// approximated: the operations on the vectors are those of two exchanges, and
+// only the FP64 sums add their terms in another order. (Left alone, one float of
+// beta off changes where the iteration stops: 2.5e-4 in a velocity at a tolerance
+// of 1e-6.)
 // The halo carries z instead of r, from which the readers form r as its owner does.
 // us an iteration with two exchanges -> one: 4.3 -> 3.6 (32^3), 5.0 -> 3.9 (64^3),
 // 6.5 -> 5.9 (96^3), 7.6 -> 7.3 (104^3). With six groups a thread the two more dot
@@ -40,8 +42,9 @@
 // exchange, at 256 bytes 2300 (writes to a line that others poll queue up).
 //
 // Arithmetic: operands, operations and their order are those of the passes
-// (k_cg_tma, k_cg_v4, k_cg_pm), so the vectors are the same bit for bit; only
-// the FP64 dot products add their terms in another order.
+// (k_cg_tma, k_cg_v4, k_cg_pm) for given alpha and beta; the FP64 dot products
+// add their terms in another order, so that once in a while an alpha or beta
+// rounds to the float beside it.
 //
 // The launch is cooperative (its CTAs wait on one another) and every wait is
 // bounded: after RES_WAIT_NS the CTA raises DONE_TIMEOUT and returns, and the
