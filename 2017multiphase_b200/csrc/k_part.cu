@@ -1084,11 +1084,12 @@ int k_correct_pos(MpCtx* c) {
     //   8                           198 181 / 1523 1390
     //   16                          610 532
     // 256^3 bubble column (8): 19.7 and 18.1 ms. Where a column of three cells is
-    // above CAP nothing is staged, and the gather has all of L1 (1200 a cell: 6.2 and
-    // 7.6 ms). Particles that have moved since the sort spread a block over cells
-    // far apart (melting block, 96^3: 0.6 and 2.0 ms).
+    // above CAP nothing is staged, and the gather has all of L1 (a heap of 1200 in its
+    // inner cells, 310 on the mean: 6.2 and 7.6 ms; 300 and 200: 2.3 and 1.4). Particles
+    // that have moved since the sort spread a block over cells far apart (melting
+    // block, 96^3: 0.6 and 2.0 ms).
     const double mean = (double)np / std::max(c->sorted_cells, 1u);
-    if (!c->moved && mean >= 6.0 && mean <= CP_CAP / 3) {
+    if (!c->moved && mean >= 6.0 && mean <= CP_CAP / 6) {
         MP_CUDA(c, cudaFuncSetAttribute(k_correct_springs, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM));
         k_correct_springs<<<mp_blocks(np, CP_T), CP_T, CP_SMEM, c->stream>>>(c->G, cells_of(c), np, c->pos, c->vel, c->pos2, re,
                                                                          P.correction_spring, P.samplespace, P.dt);
